@@ -193,6 +193,7 @@ def load():
     _proto(lib, "rvvla_last_error", C.c_char_p)
     _proto(lib, "rvvla_device_info", cint, P(cint), P(cint), P(cint))
     _proto(lib, "rvvla_kernel_launch_count", u64)
+    _proto(lib, "rvvla_trim_scratch", cint)
     _proto(lib, "rvvla_memcpy", cint, vp, vp, C.c_size_t, vp)
     _proto(lib, "rvvla_copy_h2d", cint, vp, vp, C.c_size_t, vp)
     _proto(lib, "rvvla_autotune", cint, cint, P(rvvla_crs), cint, cint, cint, P(rvvla_tune_params),

@@ -57,6 +57,38 @@ int sm_count() {
   return cache[(size_t)dev];
 }
 
+// One pool per device.  Every buffer taken from it is stream-ordered, so
+// threads and streams share it safely; the driver takes back what exceeds
+// kScratchKeep at the next synchronisation.
+static std::mutex g_pool_mu;
+static std::vector<cudaMemPool_t> g_pools;
+
+cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if ((int)g_pools.size() <= dev) g_pools.resize((size_t)dev + 1, nullptr);
+  cudaMemPool_t& pool = g_pools[(size_t)dev];
+  if (!pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kScratchKeep;
+    // making a pool is no stream operation: allowed while a stream captures
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      pool = nullptr;
+    } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaGetLastError();  // keeps nothing: slower, still correct
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  return pool;
+}
+
 }  // namespace rvvla
 
 extern "C" {
@@ -95,6 +127,18 @@ int rvvla_device_info(int* cc_major, int* cc_minor, int* sms) {
   if (cc_major) *cc_major = a;
   if (cc_minor) *cc_minor = b;
   if (sms) *sms = c;
+  return RVVLA_OK;
+}
+
+int rvvla_trim_scratch(void) {
+  int dev = 0;
+  RVVLA_CUDA(cudaGetDevice(&dev));
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(rvvla::g_pool_mu);
+    if ((int)rvvla::g_pools.size() > dev) pool = rvvla::g_pools[(size_t)dev];
+  }
+  if (pool) RVVLA_CUDA(cudaMemPoolTrimTo(pool, 0));
   return RVVLA_OK;
 }
 
