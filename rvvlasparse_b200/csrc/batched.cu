@@ -1,29 +1,45 @@
 // batched.cu — many independent SpMVs (Y_i = alpha * A_i X_i + beta * Y_i,
-// each X_i / Y_i holding k right-hand sides) in ONE persistent launch, with a
-// CUDA-graph wrapper and a measuring autotuner.  No reference counterpart.
+// each X_i / Y_i holding k right-hand sides) in one call, with a CUDA-graph
+// wrapper and a measuring autotuner.  No reference counterpart.
 //
 // Plan (rvvla_batched_plan): each matrix runs either as CSR (the caller's
 // arrays) or as SELL-C-sigma (C = 32, built on the GPU and owned by the
-// plan); its rows (CSR) or slices (SELL) are cut into tiles of bounded work,
-// and all tiles of all matrices form one list.  The kernel keeps
-// sm_count x (resident CTAs per SM) CTAs alive and walks the list with a
-// grid stride, so a batch of uneven matrices costs one launch.
+// plan).  All CSR matrices are one persistent launch over a list of tiles of
+// bounded work, all SELL matrices another over shares of slices; a plan of one
+// kind is one launch.
 //
 // Vectors: X_i is n_i x k and Y_i is m_i x k, row-major (the k values of one
 // row contiguous), packed one matrix after another; x_off/y_off give each
-// matrix's first element.  A nonzero (j, c) of row r then needs the k
-// contiguous values X[c*k .. c*k+k-1], one coalesced access per group.
+// matrix's first element.  A nonzero (j, c) of row r needs the k contiguous
+// values X[c*k .. c*k+k-1]: for k > 1, G = k * sizeof(T) / 16 lanes take 16
+// bytes each (scalars when X or Y is not 16-byte aligned).
 //
-// Mappings (per tile, one CTA of 256 threads):
-//   CSR, k = 1   tpr lanes per row (tpr in {1,2,4,...,32}, per matrix): lanes
-//                stride over the row, shuffle reduction inside the group;
-//   CSR, k > 1   k lanes per row (k in {4, 8, 32}), lane = right-hand side;
-//                the tile's columns and values (at most 2048 nonzeros) are
-//                staged in shared memory with one coalesced pass, then the
-//                group walks the row from there, each lane gathering its own
-//                X value, 8 nonzeros in flight;
-//   SELL, k = 1  a warp per slice, lane = row, column-major loads;
-//   SELL, k > 1  a warp per slice, lane = row, k accumulators per lane.
+// What bounds it: the gathers of X rows.  From L2 they come at one 32-byte
+// sector per clock and SM at best (290 G/s measured, whatever the size up to
+// 64 MB; a 128-byte row takes 1.8 clocks), from L1 at three per clock, while
+// HBM brings 2.8 fp32 nonzeros per clock and SM.
+//
+// SELL kernel: one CTA per SM, a contiguous share of the slices per CTA, so
+// that all warps of an SM work on one matrix and its X rows stay in that SM's
+// L1 (k = 1: 240 us with one CTA of 32 warps per SM, 340 with two of 16 on
+// two shares, 410 with six of 8; a window of X in shared memory left L1 too
+// few lines for the loads in flight, 301).  For rows of 32 bytes and more X
+// does not fit L1 and balance counts more: each CTA takes four shorter pieces
+// from all over the batch (k = 8: 706 -> 602 us), and 16 warps keep eight row
+// loads per lane in flight (32 warps with four: 628).
+// 256 matrices of 1K to 65K rows (0.125G nonzeros, fp32, sigma 256), tiled
+// kernel before -> now: k = 1 468 -> 242, k = 4 1024 -> 515, k = 8 2602 -> 611,
+// k = 32 16738 -> 2223 us.
+//
+// CSR kernel: a persistent grid of all the CTAs that fit walks the tiles with
+// a grid stride;
+//   k = 1   tpr lanes per row (tpr in {1,2,4,...,32}, per matrix): lanes
+//           stride over the row, shuffle reduction inside the group;
+//   k > 1   the tile's columns and values (at most 2048 nonzeros) are staged in
+//           shared memory with one coalesced pass; spr groups of G lanes per
+//           row read them from there and gather X, shuffle reduction over the
+//           groups (same batch: k = 4 918 -> 755, k = 8 1293 -> 947, k = 32 3159 ->
+//           1836 us against k lanes of one value each).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -37,7 +53,6 @@ namespace rvvla {
 namespace {
 
 constexpr int kBThreads = 256;
-constexpr int kBWarps = kBThreads / 32;
 
 struct BatchMat {
   const int* Rst;
@@ -52,12 +67,88 @@ struct BatchMat {
   const uint32_t* sPerm;
   const void* sVal;
   int64_t x_off, y_off;
-  int32_t m, n, mode, tpr;
+  int32_t m, n, mode, tpr;  // tpr: lane groups per row (CSR)
 };
 
 struct BatchTile {
   int32_t mat, first, count, pad;
 };
+
+// SELL: threads of the one CTA per SM (64 or 128 registers each), and the
+// pieces of the batch that a CTA takes.
+template <class T, int K> constexpr int kSThreads = K == 1 ? 1024 : 512;
+constexpr int kSWarpsMax = 32;
+constexpr int sell_pieces(int row_bytes) { return row_bytes >= 32 ? 4 : 1; }
+
+// A run of slices of one matrix: warp w of the CTA takes the slices
+// [first[w], first[w + 1]).
+struct BatchSeg {
+  int32_t mat, first[kSWarpsMax + 1];
+};
+
+template <class T> struct Vec16;
+template <> struct Vec16<float> { using type = float4; };
+template <> struct Vec16<double> { using type = double2; };
+
+// N values at p: one 16-byte access (VEC: p is 16-byte aligned), or scalars
+template <class T, int N, bool VEC>
+__device__ __forceinline__ void load_n(const T* p, T (&v)[N]) {
+  if constexpr (VEC && N > 1) {
+    using V = typename Vec16<T>::type;
+    static_assert(sizeof(V) == N * sizeof(T), "one 16-byte access");
+    const V t = *reinterpret_cast<const V*>(p);
+    *reinterpret_cast<V*>(v) = t;
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = p[i];
+  }
+}
+
+template <class T, int N, bool VEC>
+__device__ __forceinline__ void store_n(T* p, const T (&v)[N], T alpha, T beta) {
+  alignas(16) T o[N];
+  if (beta == T(0)) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) o[i] = alpha * v[i];
+  } else {
+    alignas(16) T y[N];
+    load_n<T, N, VEC>(p, y);
+#pragma unroll
+    for (int i = 0; i < N; ++i) o[i] = alpha * v[i] + beta * y[i];
+  }
+  if constexpr (VEC && N > 1) {
+    using V = typename Vec16<T>::type;
+    *reinterpret_cast<V*>(p) = *reinterpret_cast<const V*>(o);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[i] = o[i];
+  }
+}
+
+// X rows are gathered 16 bytes a lane (k > 1).
+template <class T, int K, bool VEC>
+struct XRows {
+  static constexpr int VPL = K == 1 ? 1 : 16 / (int)sizeof(T);  // values per lane
+  static constexpr int G = K / VPL;                             // lanes per nonzero
+};
+
+// They are re-read across a matrix: kept in L2 against the streams.
+__device__ __forceinline__ void gather16(const float* p, float (&v)[4], uint64_t pol) {
+  asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p), "l"(pol));
+}
+__device__ __forceinline__ void gather16(const double* p, double (&v)[2], uint64_t pol) {
+  asm("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v[0]), "=d"(v[1]) : "l"(p), "l"(pol));
+}
+template <class T, int N, bool VEC>
+__device__ __forceinline__ void gather_n(const T* p, T (&v)[N], uint64_t pol) {
+  if constexpr (VEC && N > 1) {
+    gather16(p, v, pol);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = ld_keep(p + i, pol);
+  }
+}
 
 template <class T>
 __device__ __forceinline__ void store_y(T* y, T alpha, T beta, T v) {
@@ -102,13 +193,14 @@ __device__ void csr_k1(const BatchMat& A, const BatchTile& t, const int* __restr
 
 constexpr int kStageNnz = 2048;  // nonzeros of a k > 1 CSR tile staged in shared memory
 
-template <class T, int K>
+template <class T, int K, bool VEC>
 __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restrict__ srst, int* __restrict__ s_col,
                        T* __restrict__ s_val, const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
-  constexpr int nslots = kBThreads / K;
-  constexpr int U = 8;
-  const int slot = threadIdx.x / K, rhs = threadIdx.x % K;
-  const T* __restrict__ x = X + A.x_off + rhs;
+  using XR = XRows<T, K, VEC>;
+  constexpr int VPL = XR::VPL, G = XR::G, U = 4;
+  const int spr = A.tpr, lanes = G * spr, nslots = kBThreads / lanes;
+  const int part = threadIdx.x % G, slot = (threadIdx.x / G) % spr, sub = threadIdx.x / lanes;
+  const T* __restrict__ x = X + A.x_off + part * VPL;
   const T* __restrict__ val = static_cast<const T*>(A.Val);
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
   const int b0 = srst[0], nzt = srst[t.count] - b0;
@@ -122,90 +214,164 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
     }
     __syncthreads();
   }
-  for (int rr = slot; rr < t.count; rr += nslots) {
-    const int b = srst[rr] - b0, e = srst[rr + 1] - b0;
-    T s[U];
+  // every group runs the same number of iterations, so the shuffles converge
+  const int iters = (t.count + nslots - 1) / nslots;
+  for (int it = 0; it < iters; ++it) {
+    const int rr = it * nslots + sub;
+    const bool valid = rr < t.count;
+    T acc[2][VPL];
 #pragma unroll
-    for (int u = 0; u < U; ++u) s[u] = T(0);
-    int j = b;
-    for (; j + U <= e; j += U) {
-      int c[U];
-      T v[U];
+    for (int i = 0; i < VPL; ++i) acc[0][i] = acc[1][i] = T(0);
+    if (valid) {
+      const int e = srst[rr + 1] - b0;
+      int j = srst[rr] - b0 + slot;
+      // rows of 128 bytes and more: whole steps, then one nonzero at a time (a
+      // repeated row would cost as much as a new one); narrower ones: idle
+      // loads of the last step repeat its first entry
+      for (; G >= 8 ? j + (U - 1) * spr < e : j < e; j += U * spr) {
+        T v[U];
+        alignas(16) T xv[U][VPL];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        c[u] = staged ? s_col[j + u] : A.Col[b0 + j + u];
-        v[u] = staged ? s_val[j + u] : val[b0 + j + u];
+        for (int u = 0; u < U; ++u) {
+          const int k = G >= 8 || j + u * spr < e ? j + u * spr : j;
+          const int c = staged ? s_col[k] : A.Col[b0 + k];
+          v[u] = staged ? s_val[k] : val[b0 + k];
+          gather_n<T, VPL, VEC>(x + (int64_t)c * K, xv[u], pl);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (G >= 8 || j + u * spr < e) {
+#pragma unroll
+            for (int i = 0; i < VPL; ++i) acc[u & 1][i] += v[u] * xv[u][i];
+          }
       }
+      for (; G >= 8 && j < e; j += spr) {
+        const int c = staged ? s_col[j] : A.Col[b0 + j];
+        const T v = staged ? s_val[j] : val[b0 + j];
+        alignas(16) T xv[VPL];
+        gather_n<T, VPL, VEC>(x + (int64_t)c * K, xv, pl);
 #pragma unroll
-      for (int u = 0; u < U; ++u) s[u] += v[u] * ld_keep(x + (int64_t)c[u] * K, pl);
+        for (int i = 0; i < VPL; ++i) acc[0][i] += v * xv[i];
+      }
     }
-    for (; j < e; ++j) {
-      const int c = staged ? s_col[j] : A.Col[b0 + j];
-      const T v = staged ? s_val[j] : val[b0 + j];
-      s[0] += v * ld_keep(x + (int64_t)c * K, pl);
-    }
-    const T r = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-    store_y(Y + A.y_off + (int64_t)(t.first + rr) * K + rhs, alpha, beta, r);
+    alignas(16) T s[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) s[i] = acc[0][i] + acc[1][i];
+    for (int off = lanes >> 1; off >= G; off >>= 1)
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], off);
+    if (valid && slot == 0)
+      store_n<T, VPL, VEC>(Y + A.y_off + (int64_t)(t.first + rr) * K + part * VPL, s, alpha, beta);
   }
 }
 
-// Slice metadata of a SELL tile (height, width, start, first sorted row),
-// staged in shared memory so a slice starts without dependent loads.
-constexpr int kTileSlicesMax = kBWarps * 4;
-
-template <class T, int K>
-__device__ void sell_kn(const BatchMat& A, const BatchTile& t, const int (*meta)[kTileSlicesMax],
-                        const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
-  constexpr int U = (K == 1) ? 8 : 4;  // columns in flight
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// One SELL slice by one warp: U columns of values and column indices are
+// loaded, then X rows, UX columns at a time.  P partial sums per row, as many
+// as the registers allow.
+template <class T, int K, bool VEC>
+__device__ __forceinline__ void sell_slice(const BatchMat& A, int sl, const T* __restrict__ x, T* __restrict__ Y,
+                                           T alpha, T beta, uint64_t pf, uint64_t pl) {
+  using XR = XRows<T, K, VEC>;
+  constexpr int VPL = XR::VPL, G = XR::G;
+  constexpr int P = K * sizeof(T) >= 128 ? 1 : K * sizeof(T) == 64 ? 2 : 4;
+  constexpr int U = G == 1 ? 8 : 4, XL = 8;  // columns, and X loads per lane, in flight
+  constexpr int UX = G == 1 ? U : XL / G > 0 ? XL / G : 1;
+  constexpr int GB = G < XL ? G : XL;
+  constexpr int RS = 32 / G;  // rows per step
+  const int lane = threadIdx.x & 31, part = lane % G;
   const T* __restrict__ val = static_cast<const T*>(A.sVal);
-  const T* __restrict__ x = X + A.x_off;
-  const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
-  for (int q = warp; q < t.count; q += kBWarps) {
-    const int h = meta[0][q], w = meta[1][q], base = meta[2][q];
-    if (lane >= h) continue;
-    const int row = (int)A.sPerm[meta[3][q] + lane];
-    T acc[K];
+  const int* __restrict__ col = reinterpret_cast<const int*>(A.sCol);
+  const int h = A.sBs[sl], w = A.sCl[sl];
+  const int mine = min(lane, h - 1);  // lanes beyond a short last slice repeat its last row
+  const int base = A.sCs[sl] + mine;
+  const int row = (int)A.sPerm[A.sSBs[sl] + mine];
+  T acc[P][G][VPL];
 #pragma unroll
-    for (int i = 0; i < K; ++i) acc[i] = T(0);
-    int j = 0;
-    for (; j + U <= w; j += U) {
-      T v[U];
-      uint32_t c[U];
+  for (int p = 0; p < P; ++p)
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t idx = (int64_t)base + (int64_t)(j + u) * h + lane;
-        v[u] = ld_stream(val + idx, pf);
-        c[u] = ld_stream(A.sCol + idx, pf);
-      }
+    for (int g = 0; g < G; ++g)
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const T* xr = x + (int64_t)c[u] * K;
+      for (int i = 0; i < VPL; ++i) acc[p][g][i] = T(0);
+  for (int j = 0; j < w; j += U) {
+    T v[U];
+    int c[U];
 #pragma unroll
-        for (int i = 0; i < K; ++i) acc[i] += v[u] * ld_keep(xr + i, pl);
+    for (int u = 0; u < U; ++u) {  // columns past the last repeat it and are not added
+      const int k = base + min(j + u, w - 1) * h;
+      v[u] = ld_stream(val + k, pf);
+      c[u] = ld_stream(col + k, pf);
+    }
+#pragma unroll
+    for (int u0 = 0; u0 < U; u0 += UX) {
+      if (u0 > 0 && j + u0 >= w) break;  // warp-uniform
+#pragma unroll
+      for (int g0 = 0; g0 < G; g0 += GB) {
+        alignas(16) T xv[UX][GB][VPL];
+        T vv[UX][GB];
+#pragma unroll
+        for (int u = 0; u < UX; ++u)
+#pragma unroll
+          for (int g = 0; g < GB; ++g) {
+            if constexpr (G == 1) {
+              vv[u][g] = v[u0 + u];
+              gather_n<T, VPL, VEC>(x + (int64_t)c[u0 + u] * K, xv[u][g], pl);
+            } else {
+              const int src = (g0 + g) * RS + lane / G;
+              const int cc = __shfl_sync(0xffffffffu, c[u0 + u], src);
+              vv[u][g] = __shfl_sync(0xffffffffu, v[u0 + u], src);
+              gather_n<T, VPL, VEC>(x + (int64_t)cc * K + part * VPL, xv[u][g], pl);
+            }
+          }
+#pragma unroll
+        for (int u = 0; u < UX; ++u)
+          if (j + u0 + u < w) {
+#pragma unroll
+            for (int g = 0; g < GB; ++g)
+#pragma unroll
+              for (int i = 0; i < VPL; ++i) acc[(u0 + u) % P][g0 + g][i] += vv[u][g] * xv[u][g][i];
+          }
       }
     }
-    for (; j < w; ++j) {
-      const int64_t idx = (int64_t)base + (int64_t)j * h + lane;
-      const T v = ld_stream(val + idx, pf);
-      const T* xr = x + (int64_t)ld_stream(A.sCol + idx, pf) * K;
+  }
 #pragma unroll
-      for (int i = 0; i < K; ++i) acc[i] += v * ld_keep(xr + i, pl);
+  for (int g = 0; g < G; ++g) {
+    alignas(16) T s[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      if constexpr (P == 4) s[i] = (acc[0][g][i] + acc[1][g][i]) + (acc[2][g][i] + acc[3][g][i]);
+      else if constexpr (P == 2) s[i] = acc[0][g][i] + acc[1][g][i];
+      else s[i] = acc[0][g][i];
     }
-    T* yr = Y + A.y_off + (int64_t)row * K;
-#pragma unroll
-    for (int i = 0; i < K; ++i) store_y(yr + i, alpha, beta, acc[i]);
+    const int rl = g * RS + lane / G;
+    const int r = G == 1 ? row : __shfl_sync(0xffffffffu, row, rl);
+    if (rl < h) store_n<T, VPL, VEC>(Y + A.y_off + (int64_t)r * K + part * VPL, s, alpha, beta);
   }
 }
 
-template <class T, int K>
+// VEC: X and Y are 16-byte aligned (k > 1; for k = 1 there is one form).
+template <class T, int K, bool VEC>
+__global__ void __launch_bounds__(kSThreads<T, K>, 1)
+batched_sell_kernel(const BatchSeg* __restrict__ segs, const int* __restrict__ share,
+                    const BatchMat* __restrict__ mats, const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
+  const int warp = threadIdx.x >> 5;
+  const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
+  const int s1 = share[blockIdx.x + 1];
+  for (int si = share[blockIdx.x]; si < s1; ++si) {  // no step of a segment spans warps
+    const BatchSeg& sg = segs[si];
+    const BatchMat& A = mats[sg.mat];
+    const int u1 = sg.first[warp + 1];
+    const T* x = X + A.x_off;
+    for (int u = sg.first[warp]; u < u1; ++u) sell_slice<T, K, VEC>(A, u, x, Y, alpha, beta, pf, pl);
+  }
+}
+
+template <class T, int K, bool VEC>
 __global__ void __launch_bounds__(kBThreads)
 batched_kernel(int64_t ntiles, const BatchTile* __restrict__ tiles, const BatchMat* __restrict__ mats,
                const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
-  // per tile: the matrix entry and the tile's row pointers (CSR) or slice
-  // metadata (SELL) are copied to shared memory once, then used by all warps
+  // per tile: the matrix entry and the tile's row pointers are copied to
+  // shared memory once, then used by all warps
   __shared__ int srst[kTileRowsMax + 1];
-  __shared__ int meta[4][kTileSlicesMax];
   __shared__ int s_col[K > 1 ? kStageNnz : 1];
   __shared__ T s_val[K > 1 ? kStageNnz : 1];
   __shared__ __align__(16) unsigned char sAraw[sizeof(BatchMat)];
@@ -218,31 +384,57 @@ batched_kernel(int64_t ntiles, const BatchTile* __restrict__ tiles, const BatchM
       reinterpret_cast<uint64_t*>(sAraw)[threadIdx.x] =
           reinterpret_cast<const uint64_t*>(mats + t.mat)[threadIdx.x];
     __syncthreads();
-    if (A.mode == 0) {  // uniform over the CTA: the tile is shared
-      for (int i = threadIdx.x; i <= t.count; i += kBThreads) srst[i] = A.Rst[t.first + i];
-      __syncthreads();
-      if constexpr (K == 1) csr_k1<T>(A, t, srst, X, Y, alpha, beta);
-      else csr_kn<T, K>(A, t, srst, s_col, s_val, X, Y, alpha, beta);
-    } else {
-      if (threadIdx.x < t.count) {
-        const int sl = t.first + threadIdx.x;
-        meta[0][threadIdx.x] = A.sBs[sl];
-        meta[1][threadIdx.x] = A.sCl[sl];
-        meta[2][threadIdx.x] = A.sCs[sl];
-        meta[3][threadIdx.x] = A.sSBs[sl];
-      }
-      __syncthreads();
-      sell_kn<T, K>(A, t, meta, X, Y, alpha, beta);
-    }
+    for (int i = threadIdx.x; i <= t.count; i += kBThreads) srst[i] = A.Rst[t.first + i];
+    __syncthreads();
+    if constexpr (K == 1) csr_k1<T>(A, t, srst, X, Y, alpha, beta);
+    else csr_kn<T, K, VEC>(A, t, srst, s_col, s_val, X, Y, alpha, beta);
   }
 }
 
-constexpr int64_t kTileWork = 8192;  // k = 1 CSR tile: nonzeros + rows; SELL tile: 4x this in products
+constexpr int64_t kTileWork = 8192;  // k = 1 CSR tile: nonzeros + rows
 
 int default_tpr(double avg) {
   int t = 1;
   while (t < 32 && t < avg) t <<= 1;
   return std::max(1, t / 2);
+}
+
+// Lanes per nonzero.
+int lanes_nz(int k, int vb) { return k == 1 ? 1 : k * vb / 16; }
+
+// Lane groups per CSR row for k > 1: at least eight nonzeros per group (fewer
+// leave more of the four loads per lane and step idle: k = 4 / 8 fp32, the
+// batch above: 907 / 1168 us with two per group, 759 / 1010 with eight).
+int default_spr(double avg, int lanes) {
+  int t = 1;
+  while (2 * t * lanes <= 32 && 16 * t <= avg) t <<= 1;
+  return t;
+}
+
+template <class T, int K, bool VEC>
+int launch_k(const rvvla_batch* B, T alpha, const T* X, T beta, T* Y, cudaStream_t st) {
+  const auto* mats = static_cast<const BatchMat*>(B->mats);
+  const auto* tiles = static_cast<const BatchTile*>(B->tiles);
+  const int64_t ncsr = B->ntiles - B->sell_segs;
+  if (ncsr > 0) {
+    batched_kernel<T, K, VEC><<<B->grid, kBThreads, 0, st>>>(ncsr, tiles, mats, X, Y, alpha, beta);
+    RVVLA_LAUNCHED("batched_kernel");
+  }
+  if (B->sell_segs > 0) {
+    const auto* segs = reinterpret_cast<const BatchSeg*>(tiles + ncsr);
+    batched_sell_kernel<T, K, VEC><<<sm_count(), kSThreads<T, K>, 0, st>>>(
+        segs, reinterpret_cast<const int*>(segs + B->sell_segs), mats, X, Y, alpha, beta);
+    RVVLA_LAUNCHED("batched_sell_kernel");
+  }
+  return RVVLA_OK;
+}
+
+template <class T, int K>
+int launch_v(const rvvla_batch* B, T alpha, const T* X, T beta, T* Y, cudaStream_t st) {
+  if constexpr (K > 1) {
+    if ((uintptr_t)X % 16 != 0 || (uintptr_t)Y % 16 != 0) return launch_k<T, K, false>(B, alpha, X, beta, Y, st);
+  }
+  return launch_k<T, K, true>(B, alpha, X, beta, Y, st);
 }
 
 template <class T>
@@ -251,26 +443,70 @@ int batched_launch(const rvvla_batch* B, T alpha, const T* X, T beta, T* Y, cuda
   if (B->val_bytes != (int)sizeof(T)) return fail(RVVLA_ERR_INVALID_ARG, "batched_spmv: value type differs from the plan");
   if (B->ntiles == 0) return RVVLA_OK;
   if ((B->x_len > 0 && !X) || (B->y_len > 0 && !Y)) return fail(RVVLA_ERR_INVALID_ARG, "batched_spmv: null vectors");
-  const auto* tiles = static_cast<const BatchTile*>(B->tiles);
-  const auto* mats = static_cast<const BatchMat*>(B->mats);
   switch (B->k) {
-    case 1: batched_kernel<T, 1><<<B->grid, kBThreads, 0, st>>>(B->ntiles, tiles, mats, X, Y, alpha, beta); break;
-    case 4: batched_kernel<T, 4><<<B->grid, kBThreads, 0, st>>>(B->ntiles, tiles, mats, X, Y, alpha, beta); break;
-    case 8: batched_kernel<T, 8><<<B->grid, kBThreads, 0, st>>>(B->ntiles, tiles, mats, X, Y, alpha, beta); break;
-    case 32: batched_kernel<T, 32><<<B->grid, kBThreads, 0, st>>>(B->ntiles, tiles, mats, X, Y, alpha, beta); break;
+    case 1: return launch_v<T, 1>(B, alpha, X, beta, Y, st);
+    case 4: return launch_v<T, 4>(B, alpha, X, beta, Y, st);
+    case 8: return launch_v<T, 8>(B, alpha, X, beta, Y, st);
+    case 32: return launch_v<T, 32>(B, alpha, X, beta, Y, st);
     default: return fail(RVVLA_ERR_INVALID_ARG, "batched_spmv: bad k in plan");
   }
-  RVVLA_LAUNCHED("batched_kernel");
-  return RVVLA_OK;
 }
 
 template <class T>
 int resident_ctas(int k) {
   int per_sm = 1;
-  auto kern = k == 1 ? batched_kernel<T, 1> : k == 4 ? batched_kernel<T, 4> : k == 8 ? batched_kernel<T, 8>
-                                                                                      : batched_kernel<T, 32>;
+  auto kern = k == 1   ? batched_kernel<T, 1, true>
+              : k == 4 ? batched_kernel<T, 4, true>
+              : k == 8 ? batched_kernel<T, 8, true>
+                       : batched_kernel<T, 32, true>;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBThreads, 0) != cudaSuccess) per_sm = 1;
   return std::max(per_sm, 1);
+}
+
+struct SliceUnit {
+  int32_t mat, slice;
+  int64_t cost;  // columns, and a share for the slice itself
+};
+
+// Cuts the slices of all SELL matrices, in order, into grid * pieces runs of
+// equal cost, gives run r to CTA r mod grid, cuts each run by matrix into
+// segments and each segment by cost over the CTA's warps.  share[c] is CTA
+// c's first segment.
+void plan_slices(const std::vector<SliceUnit>& units, int grid, int pieces, int warps, std::vector<BatchSeg>& segs,
+                 std::vector<int32_t>& share) {
+  int64_t total = 0;
+  for (const SliceUnit& u : units) total += u.cost;
+  const int64_t runs = (int64_t)grid * pieces;
+  std::vector<std::vector<BatchSeg>> per((size_t)grid);
+  int64_t done = 0;
+  size_t u0 = 0;
+  for (int64_t r = 0; r < runs; ++r) {
+    const double until = (double)total * (double)(r + 1) / (double)runs;
+    size_t u1 = u0;
+    while (u1 < units.size() && (r + 1 == runs || (double)done + 0.5 * (double)units[u1].cost < until))
+      done += units[u1++].cost;
+    while (u0 < u1) {
+      BatchSeg sg = {};
+      sg.mat = units[u0].mat;
+      size_t ue = u0;
+      int64_t cost = 0, part = 0;
+      while (ue < u1 && units[ue].mat == sg.mat) cost += units[ue++].cost;
+      const int32_t end = units[ue - 1].slice + 1;
+      for (int w = 0; w < warps; ++w) {
+        while (u0 < ue && (double)part + 0.5 * (double)units[u0].cost < (double)cost * w / warps)
+          part += units[u0++].cost;
+        sg.first[w] = u0 < ue ? units[u0].slice : end;
+      }
+      for (int w = warps; w <= kSWarpsMax; ++w) sg.first[w] = end;
+      u0 = ue;
+      per[(size_t)(r % grid)].push_back(sg);
+    }
+  }
+  share.assign((size_t)grid + 1, 0);
+  for (int c = 0; c < grid; ++c) {
+    segs.insert(segs.end(), per[(size_t)c].begin(), per[(size_t)c].end());
+    share[(size_t)c + 1] = (int32_t)segs.size();
+  }
 }
 
 // Times one plan: one warm-up launch, then the best of three (CUDA events on
@@ -307,6 +543,7 @@ int time_plan(const rvvla_batch& B, cudaStream_t st, double* ms) {
 struct BatchGraph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  int kernels = 0;
 };
 
 }  // namespace
@@ -339,6 +576,7 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
   int rc = RVVLA_OK;
   std::vector<BatchMat> tab((size_t)count);
   std::vector<BatchTile> tiles;
+  std::vector<SliceUnit> slices;
   out->x_off = static_cast<int64_t*>(std::calloc((size_t)count + 1, sizeof(int64_t)));
   out->y_off = static_cast<int64_t*>(std::calloc((size_t)count + 1, sizeof(int64_t)));
   out->sell = static_cast<rvvla_sell_owned*>(std::calloc((size_t)std::max<int64_t>(count, 1), sizeof(rvvla_sell_owned)));
@@ -379,10 +617,11 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
         rc = fail(RVVLA_ERR_INVALID_ARG, "batched_plan: threads per row must be a power of two <= 32");
         break;
       }
-      b.tpr = (k == 1) ? tpr : k;
+      b.tpr = (k == 1) ? tpr : default_spr(avg, lanes_nz(k, val_bytes));
+      const int lanes_row = (k == 1) ? tpr : b.tpr * lanes_nz(k, val_bytes);
       // tiles of whole rows: k = 1 at most kTileWork nonzeros and 8 row
       // passes of the CTA; k > 1 at most the staged nonzeros and 32 passes
-      const int64_t max_rows = std::min<int64_t>((int64_t)(kBThreads / b.tpr) * (k == 1 ? 8 : 32), kTileRowsMax);
+      const int64_t max_rows = std::min<int64_t>((int64_t)(kBThreads / lanes_row) * (k == 1 ? 8 : 32), kTileRowsMax);
       const int64_t max_work = k == 1 ? kTileWork : kStageNnz;
       int64_t r0 = 0;
       while (r0 < A.m) {
@@ -413,18 +652,7 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
         rc = fail(RVVLA_ERR_CUDA, "batched_plan: reading slice widths failed");
         break;
       }
-      int64_t q0 = 0;
-      while (q0 < s.cnt_b) {
-        int64_t q1 = q0, work = 0;
-        while (q1 < s.cnt_b && q1 - q0 < kTileSlicesMax) {
-          const int64_t wq = ((int64_t)Cl[(size_t)q1] + 1) * 32 * k;
-          if (q1 > q0 && work + wq > 4 * kTileWork) break;
-          work += wq;
-          ++q1;
-        }
-        tiles.push_back({(int32_t)i, (int32_t)q0, (int32_t)(q1 - q0), 0});
-        q0 = q1;
-      }
+      for (int64_t q = 0; q < s.cnt_b; ++q) slices.push_back({(int32_t)i, (int32_t)q, (int64_t)Cl[(size_t)q] + 2});
     } else {
       rc = fail(RVVLA_ERR_INVALID_ARG, "batched_plan: mode must be 0 (CSR) or 1 (SELL)");
       break;
@@ -442,7 +670,12 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
   h.val_bytes = val_bytes;
   h.x_len = out->x_off[count];
   h.y_len = out->y_off[count];
-  h.ntiles = (int64_t)tiles.size();
+  std::vector<BatchSeg> segs;
+  std::vector<int32_t> share;
+  plan_slices(slices, sm_count(), sell_pieces(k * val_bytes), (k == 1 ? kSThreads<float, 1> : kSThreads<float, 8>) / 32,
+              segs, share);
+  h.sell_segs = (int32_t)segs.size();
+  h.ntiles = (int64_t)(tiles.size() + segs.size());
   auto fail_cuda = [&](cudaError_t e, const char* where) {
     const int r = cuda_fail(e, where);
     std::string keep = rvvla_last_error();
@@ -453,18 +686,28 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
   cudaError_t e;
   if ((e = cudaMalloc(&out->mats, std::max<size_t>(tab.size(), 1) * sizeof(BatchMat))) != cudaSuccess)
     return fail_cuda(e, "cudaMalloc(mats)");
-  if ((e = cudaMalloc(&out->tiles, std::max<size_t>(tiles.size(), 1) * sizeof(BatchTile))) != cudaSuccess)
+  // the CSR tiles, the SELL segments and the CTAs' shares of them
+  const size_t tile_bytes = tiles.size() * sizeof(BatchTile), seg_bytes = segs.size() * sizeof(BatchSeg);
+  const size_t share_bytes = share.size() * sizeof(int32_t);
+  if ((e = cudaMalloc(&out->tiles, tile_bytes + seg_bytes + share_bytes)) != cudaSuccess)
     return fail_cuda(e, "cudaMalloc(tiles)");
   if (!tab.empty() &&
       (e = cudaMemcpyAsync(out->mats, tab.data(), tab.size() * sizeof(BatchMat), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return fail_cuda(e, "cudaMemcpyAsync(mats)");
-  if (!tiles.empty() && (e = cudaMemcpyAsync(out->tiles, tiles.data(), tiles.size() * sizeof(BatchTile),
-                                             cudaMemcpyHostToDevice, st)) != cudaSuccess)
+  char* d_tiles = static_cast<char*>(out->tiles);
+  if (!tiles.empty() &&
+      (e = cudaMemcpyAsync(d_tiles, tiles.data(), tile_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return fail_cuda(e, "cudaMemcpyAsync(tiles)");
+  if (!segs.empty() &&
+      (e = cudaMemcpyAsync(d_tiles + tile_bytes, segs.data(), seg_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+    return fail_cuda(e, "cudaMemcpyAsync(segments)");
+  if ((e = cudaMemcpyAsync(d_tiles + tile_bytes + seg_bytes, share.data(), share_bytes, cudaMemcpyHostToDevice,
+                           st)) != cudaSuccess)
+    return fail_cuda(e, "cudaMemcpyAsync(shares)");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, "cudaStreamSynchronize");
-  // persistent grid: every SM filled with as many CTAs as fit
+  // persistent grid of the CSR kernel: every SM filled with as many CTAs as fit
   const int per_sm = (val_bytes == 8) ? resident_ctas<double>(k) : resident_ctas<float>(k);
-  h.grid = (int32_t)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count() * per_sm, h.ntiles));
+  h.grid = (int32_t)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count() * per_sm, (int64_t)tiles.size()));
   h.block = kBThreads;
   h.mats = out->mats;
   h.tiles = out->tiles;
@@ -486,6 +729,7 @@ int rvvla_batched_graph(const rvvla_batch* B, double alpha, const void* X, doubl
   cudaStream_t st = as_stream(stream);
   if (!st) return fail(RVVLA_ERR_INVALID_ARG, "batched_graph: capture needs a non-default stream");
   auto* g = new BatchGraph();
+  g->kernels = (B->ntiles > B->sell_segs ? 1 : 0) + (B->sell_segs > 0 ? 1 : 0);
   const cudaError_t eb = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (eb != cudaSuccess) {
     delete g;
@@ -515,7 +759,7 @@ int rvvla_batched_graph_launch(void* graph, void* stream) {
   if (!graph) return fail(RVVLA_ERR_INVALID_ARG, "batched_graph_launch: null graph");
   auto* g = static_cast<BatchGraph*>(graph);
   RVVLA_CUDA(cudaGraphLaunch(g->exec, as_stream(stream)));
-  count_launch(1);
+  count_launch((uint64_t)g->kernels);
   return RVVLA_OK;
 }
 
