@@ -13,7 +13,7 @@
 // are skipped, lanes still holding a row at a range end get a record at the
 // next range's first vector.
 //
-// SpMV: y *= beta first (as the reference, :115-117), then one warp per
+// SpMV: y *= beta first (as the reference, :115-117), then the warps of each
 // range (lane = CVR lane): coalesced 32-wide vector loads (L2 evict-first),
 // x gathers (evict-last), and per batch of vectors the records that fall in
 // it are scattered to their (vector, lane) slots through a shared table; a
@@ -169,36 +169,75 @@ __global__ void cvr_scale_kernel(int64_t m, X* __restrict__ y, X beta) {
   if (i < m) y[i] = (beta == X(0)) ? X(0) : y[i] * beta;
 }
 
-// A warp per CVR thread (lane = SIMD lane), cvr_batch<V>() vectors per batch.  A
-// batch first issues all loads of its vectors (indices past the range are
-// clamped to its last vector and their products dropped), then marks the
-// records that fall in the batch in a per-warp table (vector in batch, lane)
-// -> row, then each lane walks the batch's vectors: flush into the marked row
-// (the record's position is the lane's first slot after the row), add the
-// product.  Records come from a 32-entry register window (lane l holds
-// record window_base + l) with the next window prefetched.  A row belongs to
-// one lane of one range, so each row of y receives exactly one contribution:
-// y was scaled by beta first and the flush is a fire-and-forget atomic add
-// (no read of y on the critical path, and still deterministic).  Vectors per
-// batch: 8 for 8-byte values, 16 for 4-byte ones (about the same bytes in
-// flight).
-template <class V> constexpr int cvr_batch() { return sizeof(V) >= 8 ? 8 : 16; }
+// A CVR range is shared by kCvrSplit warps (lane = SIMD lane), warp i taking
+// the i-th share of its vectors in batches of kCvrBatch vectors.  A batch
+// first issues all loads of its vectors (indices past the share are clamped to
+// its last vector and their products dropped), then marks the records that
+// fall in the batch in a per-warp table (vector in batch, lane) -> row, then
+// each lane walks the batch's vectors: flush into the marked row (the record's
+// position is the lane's first slot after the row), add the product.  Records
+// come from a 32-entry register window (lane l holds record window_base + l)
+// with the next window prefetched; a warp finds its first record by a 32-ary
+// search.  A row belongs to one lane of one range: rows that begin and end in
+// one share are flushed there, and a lane's sum before its first flush of a
+// later share (the row crosses into it) is kept for the range's first warp,
+// which adds a row's pieces in share order.  So each row of y receives exactly
+// one contribution: y was scaled by beta first and the flush is a
+// fire-and-forget atomic add (no read of y on the critical path, and still
+// deterministic).
+//
+// Why the split: a range of 16K nonzeros per warp left 8 warps per SM on a
+// matrix of 20M nonzeros (random rows, n = 2^20, fp64: 188 us with one warp per
+// range, 144 / 127 / 120 with two / four / eight; fp32 118 -> 96; the
+// 67M-nonzero power-law matrix 527 -> 321 us fp64, 405 -> 246 fp32; 1.6M
+// nonzeros 133 -> 33 us fp64), while smaller ranges would pad the format.
+// Bound by the gathers from L2 (one a clock and SM: 69 us for the random
+// matrix).  fp32 runs four CTAs per SM with batches of 8 (three with batches of
+// 16: 116 us), fp64 three (four spill: 133).
+constexpr int kCvrSplit = 8;
+constexpr int kCvrBatch = 8;
 
 template <class V, class X, class CT>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(256, sizeof(V) >= 8 ? 3 : 4)
 cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ vals,
                 const uint32_t* __restrict__ cols, const int* __restrict__ rec, const int* __restrict__ wb,
                 const X* __restrict__ x, X* __restrict__ y, X alpha) {
-  constexpr int kCvrU = cvr_batch<V>();
+  constexpr int kCvrU = kCvrBatch;
+  constexpr int kRanges = 8 / kCvrSplit;  // ranges per CTA
   __shared__ int s_row[8][kCvrU][kS];
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  __shared__ int s_head_row[8][kS];  // per share and lane: row of the first flush (-1: none), the sum
+  __shared__ CT s_head[8][kS];       // before it, and the sum after the last one
+  __shared__ CT s_tail[8][kS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (t >= NT) return;
-  const int64_t vb = wb[t * (kS + 2)], rb = wb[t * (kS + 2) + 1];
-  const int64_t ve = (t + 1 < NT) ? wb[(t + 1) * (kS + 2)] : nItems / kS;
-  const int64_t re = (t + 1 < NT) ? wb[(t + 1) * (kS + 2) + 1] : nrec;
+  const int64_t t = (int64_t)blockIdx.x * kRanges + w / kCvrSplit;
+  const int part = w % kCvrSplit;
+  const bool last = part == kCvrSplit - 1;
+  int64_t vb = 0, ve = 0, rb = 0, re = 0;
+  if (t < NT) {
+    vb = wb[t * (kS + 2)];
+    rb = wb[t * (kS + 2) + 1];
+    ve = (t + 1 < NT) ? wb[(t + 1) * (kS + 2)] : nItems / kS;
+    re = (t + 1 < NT) ? wb[(t + 1) * (kS + 2) + 1] : nrec;
+    const int64_t nv = ve - vb;
+    ve = vb + nv * (part + 1) / kCvrSplit;
+    vb += nv * part / kCvrSplit;
+    if (part > 0) {  // first record at or after the share's first vector: rec[2 * rb] < it <= rec[2 * hi]
+      int64_t lo = rb - 1, hi = re;
+      while (hi - lo > 1) {
+        const int64_t step = (hi - lo + kS - 1) / kS;
+        const int64_t at = lo + step * (lane + 1);
+        const bool before = at < hi && rec[2 * at] < vb * kS;
+        const int k = __popc(__ballot_sync(0xffffffffu, before));  // positions rise: a prefix of the lanes
+        hi = min(hi, lo + step * (k + 1));
+        lo += step * k;
+      }
+      rb = hi;
+    }
+  }
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
   CT res = 0;
+  bool open = part > 0;  // no flush yet in this share: the sum may continue an earlier share's row
+  s_head_row[w][lane] = -1;
 #pragma unroll
   for (int u = 0; u < kCvrU; ++u) s_row[w][u][lane] = -1;
   // record window and its successor
@@ -242,7 +281,13 @@ cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ 
     for (int u = 0; u < kCvrU; ++u) {
       const int r = s_row[w][u][lane];
       if (r >= 0) {
-        if (res != CT(0)) atomicAdd(y + r, alpha * (X)res);
+        if (open) {
+          s_head_row[w][lane] = r;
+          s_head[w][lane] = res;
+          open = false;
+        } else if (res != CT(0)) {
+          atomicAdd(y + r, alpha * (X)res);
+        }
         res = 0;
         s_row[w][u][lane] = -1;
       }
@@ -261,7 +306,7 @@ cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ 
     for (int u = 0; u < kCvrU; ++u) a[u] = ld_stream(vals + min(v + u, ve - 1) * kS + lane, pf);
 #pragma unroll
     for (int u = 0; u < kCvrU; ++u) xv[u] = ld_keep(x + c[u], pl);
-    mark((v + kCvrU) * kS, v);
+    mark((last || v + kCvrU < ve ? v + kCvrU : ve) * kS, v);
     CT p[kCvrU];
 #pragma unroll
     for (int u = 0; u < kCvrU; ++u) p[u] = (CT)vmul(a[u], xv[u]);
@@ -272,7 +317,7 @@ cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ 
   CT none[kCvrU];
 #pragma unroll
   for (int u = 0; u < kCvrU; ++u) none[u] = 0;
-  for (int guard = 0; guard < 64; ++guard) {
+  for (int guard = 0; last && guard < 64; ++guard) {
     if (cons == navail && navail < kS) break;
     const int64_t p0 = __shfl_sync(0xffffffffu, my_pos, cons < kS ? cons : 0);
     if (cons == navail) {  // window used up: reload through mark
@@ -284,9 +329,24 @@ cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ 
     flush_batch(0, none);
     v += kCvrU;
   }
+  s_tail[w][lane] = res;
+  __syncthreads();
+  if (part != 0 || t >= NT) return;
+  // rows that cross shares: the pieces of a lane in share order
+  CT sum = res;
+  for (int i = 1; i < kCvrSplit; ++i) {
+    const int r = s_head_row[w + i][lane];
+    if (r >= 0) {
+      sum += s_head[w + i][lane];
+      if (sum != CT(0)) atomicAdd(y + r, alpha * (X)sum);
+      sum = s_tail[w + i][lane];
+    } else {
+      sum += s_tail[w + i][lane];
+    }
+  }
   if (t + 1 == NT) {  // the last range's tail rows
     const int r = wb[t * (kS + 2) + 2 + lane];
-    if (res != CT(0)) atomicAdd(y + r, alpha * (X)res);
+    if (sum != CT(0)) atomicAdd(y + r, alpha * (X)sum);
   }
 }
 
@@ -308,7 +368,7 @@ int cvr_spmv_impl(const rvvla_cvr* A, X alpha, const X* x, X beta, X* y, cudaStr
   RVVLA_LAUNCHED("cvr_scale_kernel");
   const int64_t NT = A->Nthreads_avail;
   const int64_t nrec = (A->n_record - 2) / 2;
-  cvr_spmv_kernel<V, X, CT><<<(unsigned)((NT * 32 + 255) / 256), 256, 0, st>>>(
+  cvr_spmv_kernel<V, X, CT><<<(unsigned)((NT * kCvrSplit + 7) / 8), 256, 0, st>>>(
       NT, A->nItems, nrec, (const V*)A->vPack_vec_vals, A->vPack_vec_cols, A->vPack_vec_record,
       A->writeback_pos_record, x, y, alpha);
   RVVLA_LAUNCHED("cvr_spmv_kernel");
