@@ -68,45 +68,102 @@ __global__ void tr_gather_kernel(int64_t nz, const int* __restrict__ perm, const
 }
 
 constexpr int kSdThreads = 256;
-constexpr int kSdRows = 256;  // rows per CTA
-constexpr int kSdU = 4;       // nonzeros per thread in flight
+constexpr int kSdRows = 256;    // rows per CTA
+constexpr int kSdChunk = 4096;  // nonzeros per pass over the row-start bitmap
+constexpr int kSdU = 8;         // nonzeros per thread in flight
 
-// dv[k] = g[row(k)] * x[Col[k]]: a CTA per 256 consecutive rows, their row
-// pointers staged in shared memory (no search in global memory); each thread
-// takes every 256th nonzero of the CTA's range, finds its row by binary
-// search over the staged pointers and keeps 4 nonzeros' loads in flight.
+// dv[k] = g[row(k)] * x[Col[k]]: a CTA per 256 consecutive rows.  The g of its
+// non-empty rows are compacted into shared memory; a bitmap marks the
+// nonzeros of a chunk that start a non-empty row, with the count of marks
+// before each of its words, so a nonzero's row is one popcount away (a warp's
+// 32 nonzeros are one word).  The chunks start at multiples of 32.
+//
+// Bound by the gathers of x: random columns reach L2 at one 32-byte sector per
+// clock and SM at best, 69 us for 19.9M nonzeros over 2^20 columns, fp32; this
+// takes 97 us, a binary search per nonzero over staged row pointers took 117 (fp64 107, 126).
 template <class T>
 __global__ void __launch_bounds__(kSdThreads)
 sddmm_kernel(int64_t m, const int* __restrict__ Rst, const int* __restrict__ Col, const T* __restrict__ g,
              const T* __restrict__ x, T* __restrict__ dv) {
-  __shared__ int win[kSdRows + 1];
+  constexpr int W = kSdChunk / 32;
+  __shared__ int s_start[kSdRows];  // first nonzero of each non-empty row
+  __shared__ T s_g[kSdRows];
+  __shared__ unsigned s_bits[W];
+  __shared__ int s_before[W];
+  __shared__ int s_sum[kSdThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * kSdRows;
   const int nr = (int)min((int64_t)kSdRows, m - r0);
-  for (int i = threadIdx.x; i <= nr; i += kSdThreads) win[i] = Rst[r0 + i];
+  const int kb = Rst[r0], ke = Rst[r0 + nr];
+  // compact the non-empty rows in row order
+  const int b = t < nr ? Rst[r0 + t] : 0, e = t < nr ? Rst[r0 + t + 1] : 0;
+  const bool full = e > b;
+  const unsigned fulls = __ballot_sync(0xffffffffu, full);
+  if (lane == 0) s_sum[warp] = __popc(fulls);
   __syncthreads();
-  const int kb = win[0], ke = win[nr];
+  int at = __popc(fulls & ((1u << lane) - 1u)), rows = 0;
+#pragma unroll
+  for (int i = 0; i < kSdThreads / 32; ++i) {
+    if (i < warp) at += s_sum[i];
+    rows += s_sum[i];
+  }
+  if (full) {
+    s_start[at] = b;
+    s_g[at] = g[r0 + t];
+  }
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
-  for (int k0 = kb + (int)threadIdx.x; k0 < ke; k0 += kSdU * kSdThreads) {
-    int c[kSdU];
-    T gv[kSdU];
+  for (int c0 = kb / 32 * 32; c0 < ke; c0 += kSdChunk) {
+    if (t < W) s_bits[t] = 0u;
+    __syncthreads();
+    int earlier = 0;  // non-empty rows that start before the chunk
+    if (t < rows) {
+      const int k = s_start[t] - c0;
+      earlier = k < 0;
+      if (k >= 0 && k < kSdChunk) atomicOr(&s_bits[k >> 5], 1u << (k & 31));
+    }
+    earlier = __syncthreads_count(earlier);
+    // marks before each word: warps 0 .. W / 32 - 1 scan 32 words each
+    int cnt = 0, inc = 0;
+    if (t < W) {
+      cnt = inc = __popc(s_bits[t]);
 #pragma unroll
-    for (int u = 0; u < kSdU; ++u) {
-      const int k = min(k0 + u * kSdThreads, ke - 1);
-      int lo = 0, hi = nr - 1;  // largest j with win[j] <= k
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (win[mid] <= k) lo = mid;
-        else hi = mid - 1;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += o;
       }
-      c[u] = ld_stream(Col + k, pf);
-      gv[u] = g[r0 + lo];
+      if (lane == 31) s_sum[warp] = inc;
     }
+    __syncthreads();
+    if (t < W) {
+      int base = earlier + inc - cnt;
+      for (int i = 0; i < warp; ++i) base += s_sum[i];
+      s_before[t] = base;
+    }
+    __syncthreads();
+    const int end = min(ke - c0, kSdChunk);
+    for (int k0 = t; k0 < end; k0 += kSdU * kSdThreads) {
+      int c[kSdU];
+      T gv[kSdU], xv[kSdU];
 #pragma unroll
-    for (int u = 0; u < kSdU; ++u) {
-      const int k = k0 + u * kSdThreads;
-      const T xv = ld_keep(x + c[u], pl);
-      if (k < ke) dv[k] = gv[u] * xv;
+      for (int u = 0; u < kSdU; ++u) {  // loads past the chunk's range repeat its last nonzero
+        const int k = min(k0 + u * kSdThreads, end - 1);
+        c[u] = ld_stream(Col + max(c0 + k, kb), pf);
+      }
+#pragma unroll
+      for (int u = 0; u < kSdU; ++u) {
+        const int k = min(k0 + u * kSdThreads, end - 1);
+        const int i = s_before[k >> 5] + __popc(s_bits[k >> 5] & ((2u << (k & 31)) - 1u)) - 1;
+        gv[u] = s_g[max(i, 0)];  // (nonzeros before the CTA's first: not stored)
+      }
+#pragma unroll
+      for (int u = 0; u < kSdU; ++u) xv[u] = ld_keep(x + c[u], pl);
+#pragma unroll
+      for (int u = 0; u < kSdU; ++u) {
+        const int k = k0 + u * kSdThreads;
+        if (k < end && c0 + k >= kb) dv[c0 + k] = gv[u] * xv[u];
+      }
     }
+    __syncthreads();  // the bitmap is read
   }
 }
 
