@@ -29,7 +29,7 @@
  *   - Entry points that need temporary device memory obtain it stream-ordered
  *     on `stream`, from a memory pool of the library's own (the ordinary fp64
  *     CSR5 entry: from the device's default pool).  Between calls that pool
- *     keeps at most 64 MB per device; rvvla_trim_scratch() gives it back.
+ *     keeps at most 256 MB per device; rvvla_trim_scratch() gives it back.
  */
 #ifndef RVVLA_H
 #define RVVLA_H
@@ -75,7 +75,7 @@ int rvvla_device_info(int* cc_major, int* cc_minor, int* sm_count);
 /* Number of kernels this library launched in this process (all entry points). */
 uint64_t rvvla_kernel_launch_count(void);
 /* Returns the unused temporary memory that the library's pool on the current
- * device keeps between calls (at most 64 MB) to the driver. */
+ * device keeps between calls (at most 256 MB) to the driver. */
 int rvvla_trim_scratch(void);
 /* cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream) followed by a
  * stream synchronisation; for callers that manage memory themselves (the

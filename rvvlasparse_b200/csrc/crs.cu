@@ -156,20 +156,60 @@ int crs_plan_launch(int64_t m, int64_t nz, const int32_t* Rst, int ipt, int32_t*
   return RVVLA_OK;
 }
 
+// The fix-up after a lane-run launch with dot partials, and their sum: block b
+// adds the partials of its 128 warps, and the block that finishes last adds
+// the blocks' sums, in block order, into *dot.  `ticket` is 0 before and after.
+template <class X, class CT>
+__global__ void __launch_bounds__(256)
+crs_dot_fixup_kernel(int nw, const int* __restrict__ carry_row, const CT* __restrict__ carry_val, X* __restrict__ y,
+                     X alpha, X beta, const int* __restrict__ row_map, const CT* __restrict__ part,
+                     double* __restrict__ sums, unsigned* __restrict__ ticket, double* __restrict__ dot) {
+  __shared__ double sh[256];
+  __shared__ bool last;
+  const int t = threadIdx.x;
+  grid_chain();
+  crs_fixup_slot((int)(blockIdx.x * 256 + t), 2 * nw, carry_row, carry_val, y, alpha, beta, row_map);
+  const int w = blockIdx.x * 128 + t;
+  sh[t] = t < 128 && w < nw ? (double)part[w] : 0.0;
+  __syncthreads();
+  for (int d = 64; d > 0; d >>= 1) {
+    if (t < d) sh[t] += sh[t + d];
+    __syncthreads();
+  }
+  if (t == 0) {
+    sums[blockIdx.x] = sh[0];
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0;
+  for (int i = t; i < (int)gridDim.x; i += 256) a += __ldcg(sums + i);
+  sh[t] = a;
+  __syncthreads();
+  for (int d = 128; d > 0; d >>= 1) {
+    if (t < d) sh[t] += sh[t + d];
+    __syncthreads();
+  }
+  if (t == 0) {
+    *dot = sh[0];
+    *ticket = 0u;
+  }
+}
+
 // perm/pval (the adjoint): value k of A is pval[perm[k]]; needs an analysed
 // plan (kinds 1 and 2) when A has nonzeros.
-// dot_part (the solvers): the lane-run kernel also writes one partial of
-// x^T (y - beta y) / alpha per warp (see crs_run_kernel), *nparts of them
-// (at most dot_cap); needs an analysed plan.
+// dot (the solvers): the lane-run kernel also writes one partial of
+// x^T (y - beta y) / alpha per warp (see crs_run_kernel), and the fix-up adds
+// them into *dot->out; needs an analysed plan and nonzeros.
 template <class V, class X, class Ac, class P, class CT, int IPT>
 int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStream_t st,
-                  const int32_t* perm = nullptr, const V* pval = nullptr, CT* dot_part = nullptr,
-                  int64_t dot_cap = 0, int64_t* nparts = nullptr) {
+                  const int32_t* perm = nullptr, const V* pval = nullptr, const CrsDot* dot = nullptr) {
   int rc = crs_validate(A, x, y);
   if (rc) return rc;
-  if (nparts) *nparts = 0;
   if (A->m == 0) return RVVLA_OK;
-  if ((perm || dot_part) && A->nz > 0 && !(A->plan && (A->plan_kind == 1 || A->plan_kind == 2)))
+  if ((perm || dot) && A->nz > 0 && !(A->plan && (A->plan_kind == 1 || A->plan_kind == 2)))
     return fail(RVVLA_ERR_INVALID_ARG, "crs: this product needs an analysed plan (rvvla_crs_analyze)");
   if (A->plan && (A->plan_kind == 1 || A->plan_kind == 2)) {  // shared-memory-free stream kernel
     // kind 1: plan_tiles = warps, all rows; kind 2: plan_tiles = number of
@@ -203,19 +243,13 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
     int32_t* crow = sc.as<int32_t>();
     CT* cval = (CT*)(sc.as<char>() + row_bytes);
     const unsigned blocks = (unsigned)((nw * 32 + 255) / 256);
+    CT* dot_part = dot ? reinterpret_cast<CT*>(dot->part) : nullptr;
     if (dot_part) {
-      if (nw > dot_cap) return fail(RVVLA_ERR_TOO_LARGE, "crs: dot partial buffer too small");
-      *nparts = nw;
       const bool vec = (uintptr_t)A->Col % 16 == 0 && (uintptr_t)A->Val % 16 == 0;
-      if (vec)
-        crs_run_kernel<V, X, Ac, CT, true, false, true><<<blocks, 256, 0, st>>>(
-            mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, (const V*)A->Val, x, y, alpha, beta, wrow, crow, cval,
-            row_map, nullptr, dot_part);
-      else
-        crs_run_kernel<V, X, Ac, CT, false, false, true><<<blocks, 256, 0, st>>>(
-            mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, (const V*)A->Val, x, y, alpha, beta, wrow, crow, cval,
-            row_map, nullptr, dot_part);
-      RVVLA_LAUNCHED("crs_run_kernel");
+      auto kern = vec ? crs_run_kernel<V, X, Ac, CT, true, false, true> : crs_run_kernel<V, X, Ac, CT, false, false, true>;
+      RVVLA_CUDA(launch_chained(kern, blocks, 256, st, mr, (int)A->nz, E, (int)nw, rst, bits, A->Col,
+                                (const V*)A->Val, x, y, alpha, beta, wrow, crow, cval, row_map, nullptr, dot_part));
+      count_launch();
     } else if (perm) {
       const bool vec = (uintptr_t)A->Col % 16 == 0 && (uintptr_t)perm % 16 == 0;
       if (vec)
@@ -244,9 +278,15 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
                                                                     crow, cval, row_map);
       RVVLA_LAUNCHED("crs_run_kernel");
     }
-    crs_stream_fixup_kernel<X, CT><<<(unsigned)((2 * nw + 255) / 256), 256, 0, st>>>((int)(2 * nw), crow, cval, y,
-                                                                                       alpha, beta, row_map);
-    RVVLA_LAUNCHED("crs_stream_fixup_kernel");
+    const unsigned fix_blocks = (unsigned)((2 * nw + 255) / 256);
+    if (dot) {
+      RVVLA_CUDA(launch_chained(crs_dot_fixup_kernel<X, CT>, fix_blocks, 256, st, (int)nw, crow, cval, y, alpha, beta,
+                                row_map, dot_part, dot->sums, dot->ticket, dot->out));
+      count_launch();
+    } else {
+      crs_stream_fixup_kernel<X, CT><<<fix_blocks, 256, 0, st>>>((int)(2 * nw), crow, cval, y, alpha, beta, row_map);
+      RVVLA_LAUNCHED("crs_stream_fixup_kernel");
+    }
     return RVVLA_OK;
   }
   const int64_t nt = crs_tiles(A->m, A->nz, IPT);
@@ -275,17 +315,14 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
   return RVVLA_OK;
 }
 
-// q = A p with the fused dot (alpha 1, beta 0): part[0..*nparts) sum to
-// p^T A p; used by the solvers.
-int crs_spmv_dot_f64(const rvvla_crs* A, const double* p, double* q, double* part, int64_t cap, int64_t* nparts,
-                     cudaStream_t st) {
+// q = A p and *dot.out = p^T A p (alpha 1, beta 0); used by the solvers.
+int crs_spmv_dot_f64(const rvvla_crs* A, const double* p, double* q, const CrsDot& dot, cudaStream_t st) {
   return crs_spmv_impl<double, double, double, double, double, MergeCfg<double>::IPT>(A, 1.0, p, 0.0, q, st, nullptr,
-                                                                                      nullptr, part, cap, nparts);
+                                                                                      nullptr, &dot);
 }
-int crs_spmv_dot_f32(const rvvla_crs* A, const float* p, float* q, float* part, int64_t cap, int64_t* nparts,
-                     cudaStream_t st) {
+int crs_spmv_dot_f32(const rvvla_crs* A, const float* p, float* q, const CrsDot& dot, cudaStream_t st) {
   return crs_spmv_impl<float, float, float, float, float, MergeCfg<float>::IPT>(A, 1.0f, p, 0.0f, q, st, nullptr,
-                                                                               nullptr, part, cap, nparts);
+                                                                               nullptr, &dot);
 }
 int64_t crs_warp_count(int64_t nz) {
   const int E = crs_warp_span(nz);

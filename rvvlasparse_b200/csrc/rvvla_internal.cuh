@@ -60,7 +60,7 @@ cudaMemPool_t scratch_pool();
 // synchronisation mapped its few KB of carries anew (the CRS fp64 product of
 // 4M power-law rows, first call on a new matrix: 883 us, 406 us with this
 // pool).  Larger buffers (builders) come from the default pool as before.
-constexpr uint64_t kScratchKeep = 64ull << 20;
+constexpr uint64_t kScratchKeep = 256ull << 20;  // a solve on 8M rows in fp64 fits
 struct Scratch {
   void* p = nullptr;
   cudaStream_t s = nullptr;
@@ -82,6 +82,42 @@ struct Scratch {
   template <class T>
   T* as() const { return reinterpret_cast<T*>(p); }
 };
+
+// Buffers of the CRS product with a fused dot (crs.cu; the solvers').  part:
+// one entry of the value type per warp, sums: one double per 128 warps,
+// ticket: 0 before and after a product, out: the dot.
+struct CrsDot {
+  void* part;
+  double* sums;
+  unsigned* ticket;
+  double* out;
+};
+
+// Launches that may start while the stream's previous kernel drains: the
+// kernel calls grid_chain() before it touches anything that kernel writes or
+// reads.  In a chain of short kernels this hides the launch and the ramp-up.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// By every CTA that does any work: lets the stream's next chained kernel start
+// once all CTAs have come here, and waits until the previous kernel is
+// complete and its writes are visible.  Neither does anything in a kernel
+// launched the ordinary way.
+__device__ __forceinline__ void grid_chain() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // ------------------------------------------------------------------ loads
 // Streaming operands (values, indices) are read once: evict-first in L2 and

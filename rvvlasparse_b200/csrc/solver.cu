@@ -2,16 +2,21 @@
 // BiCGStab (general square A) over the CRS kernels (no reference
 // counterpart: callers of the SpMV path).
 //
-// A CG iteration is five launches on the caller's stream and no host
+// A CG iteration is four launches on the caller's stream and no host
 // synchronisation:
 //   1. q = A p with the fused dot: the CRS lane-run kernel adds p[row] * v
 //      for every row piece v it stores or carries into a per-warp partial,
 //      so p^T A p needs no second pass over q;
-//   2. one block sums the partials (fixed order) and sets alpha = r.r / p.q;
-//   3. x += alpha p, r -= alpha q and per-block partials of the new r.r in
-//      the same pass (the axpy/dot epilogue fused);
-//   4. one block sums them and sets beta = r.r(new) / r.r(old);
-//   5. p = r + beta p.
+//   2. the rows that cross warps, and the sum of those partials: p.q;
+//   3. r -= alpha q with alpha = r.r / p.q, and the new r.r in the same pass;
+//   4. x += alpha p and p = r + beta p, beta = r.r(new) / r.r(old), one read of
+//      p for both.
+// (2) and (3) add their blocks' partials in the block that finishes last.
+// Bound by HBM: the product (see crs_run.cuh) and 8 vectors a pass.  5-point
+// Laplacian 2048^2, fp64: 167 us per iteration with the scalars in kernels of
+// their own and x updated beside r (9 vectors), 155 with four launches, 147
+// with each launch chained to the one before (grid_chain: it starts while that
+// one drains).
 // The scalars live in device memory; every check_every iterations the host
 // reads r.r once to test ||r|| <= rtol ||b||.  All reductions run in a fixed
 // order, so a solve is bitwise reproducible.
@@ -24,19 +29,17 @@
 
 namespace rvvla {
 
-int crs_spmv_dot_f64(const rvvla_crs* A, const double* p, double* q, double* part, int64_t cap, int64_t* nparts,
-                     cudaStream_t st);
-int crs_spmv_dot_f32(const rvvla_crs* A, const float* p, float* q, float* part, int64_t cap, int64_t* nparts,
-                     cudaStream_t st);
+int crs_spmv_dot_f64(const rvvla_crs* A, const double* p, double* q, const CrsDot& dot, cudaStream_t st);
+int crs_spmv_dot_f32(const rvvla_crs* A, const float* p, float* q, const CrsDot& dot, cudaStream_t st);
 int64_t crs_warp_count(int64_t nz);
 
 namespace {
 
 struct CgScalars {
-  double rr;      // r.r of the current residual
-  double pq;      // p.(A p)
-  double alpha, beta;
-  double bb;      // b.b
+  double rr[2];  // r.r of the residuals of even and odd iterations
+  double pq;     // p.(A p)
+  double bb;     // b.b
+  unsigned ticket_dot, ticket_rr;  // blocks done, of the kernels that add partials (0 between launches)
 };
 
 constexpr int kRedThreads = 1024;
@@ -56,24 +59,6 @@ __device__ double block_sum(const T* __restrict__ v, int64_t n) {
     __syncthreads();
   }
   return sh[0];
-}
-
-template <class T>
-__global__ void __launch_bounds__(kRedThreads) cg_alpha_kernel(const T* __restrict__ part, int64_t n, CgScalars* s) {
-  const double pq = block_sum(part, n);
-  if (threadIdx.x == 0) {
-    s->pq = pq;
-    s->alpha = pq != 0.0 ? s->rr / pq : 0.0;
-  }
-}
-
-__global__ void __launch_bounds__(kRedThreads) cg_beta_kernel(const double* __restrict__ part, int64_t n,
-                                                              CgScalars* s) {
-  const double rr = block_sum(part, n);
-  if (threadIdx.x == 0) {
-    s->beta = s->rr != 0.0 ? rr / s->rr : 0.0;
-    s->rr = rr;
-  }
 }
 
 // per-block partial of u.v over a grid-stride loop (fixed grid: fixed order)
@@ -101,25 +86,84 @@ __global__ void __launch_bounds__(kRedThreads) cg_set_kernel(const double* __res
                                                              CgScalars* s, int which) {
   const double v = block_sum(part, n);
   if (threadIdx.x == 0) {
-    if (which == 0) s->rr = v;
-    else s->bb = v;
+    if (which == 0) {
+      s->rr[0] = v;
+      s->ticket_dot = s->ticket_rr = 0u;
+    } else {
+      s->bb = v;
+    }
   }
 }
 
+__device__ __forceinline__ double cg_alpha(const CgScalars* s, int cur) {
+  return s->pq != 0.0 ? s->rr[cur] / s->pq : 0.0;
+}
+
+// r -= alpha q and the new r.r: the block that finishes last adds the blocks'
+// partials in a fixed order.
 template <class T>
-__global__ void __launch_bounds__(kUpdThreads) cg_update_kernel(int64_t n, T* __restrict__ x, T* __restrict__ r,
-                                                                const T* __restrict__ p, const T* __restrict__ q,
-                                                                const CgScalars* __restrict__ s,
-                                                                double* __restrict__ part) {
-  const T alpha = (T)s->alpha;
+__global__ void __launch_bounds__(kUpdThreads) cg_update_kernel(int64_t n, T* __restrict__ r, const T* __restrict__ q,
+                                                                CgScalars* s, int cur, double* part) {
+  __shared__ bool last;
+  grid_chain();
+  // r and q start 16-byte aligned: 16 bytes a thread, two loads of each in flight
+  constexpr int E = 16 / (int)sizeof(T);
+  struct alignas(16) Vec {
+    T v[E];
+  };
+  const T alpha = (T)cg_alpha(s, cur);
   double a = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * kUpdThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kUpdThreads) {
-    x[i] += alpha * p[i];
-    const T ri = r[i] - alpha * q[i];
-    r[i] = ri;
-    a += (double)ri * (double)ri;
+  const int64_t nv = n / E, step = (int64_t)gridDim.x * kUpdThreads;
+  Vec* rv = reinterpret_cast<Vec*>(r);
+  const Vec* qv = reinterpret_cast<const Vec*>(q);
+  auto upd = [&](Vec& ri, const Vec& qi) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      ri.v[e] -= alpha * qi.v[e];
+      a += (double)ri.v[e] * (double)ri.v[e];
+    }
+  };
+  int64_t i = (int64_t)blockIdx.x * kUpdThreads + threadIdx.x;
+  for (; i + step < nv; i += 2 * step) {
+    Vec r0 = rv[i], r1 = rv[i + step];
+    const Vec q0 = qv[i], q1 = qv[i + step];
+    upd(r0, q0);
+    upd(r1, q1);
+    rv[i] = r0;
+    rv[i + step] = r1;
+  }
+  if (i < nv) {
+    Vec r0 = rv[i];
+    upd(r0, qv[i]);
+    rv[i] = r0;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < n - nv * E) {  // the last n mod E
+    const int64_t k = nv * E + threadIdx.x;
+    const T rk = r[k] - alpha * q[k];
+    r[k] = rk;
+    a += (double)rk * (double)rk;
   }
   block_partial(a, part);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&s->ticket_rr, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kUpdThreads) t += __ldcg(part + i);
+  __shared__ double sh[kUpdThreads];
+  sh[threadIdx.x] = t;
+  __syncthreads();
+  for (int d = kUpdThreads / 2; d > 0; d >>= 1) {
+    if ((int)threadIdx.x < d) sh[threadIdx.x] += sh[threadIdx.x + d];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    s->rr[cur ^ 1] = sh[0];
+    s->ticket_rr = 0u;
+  }
 }
 
 template <class T>
@@ -127,6 +171,11 @@ __global__ void __launch_bounds__(kRedThreads) sum_to_kernel(const T* __restrict
   const double v = block_sum(part, n);
   if (threadIdx.x == 0) *out = (T)v;
 }
+
+template <class T>
+__global__ void store_dot_kernel(const double* __restrict__ v, T* __restrict__ out) { *out = (T)*v; }
+
+int64_t dot_blocks(int64_t nw) { return (2 * nw + 255) / 256; }  // crs_dot_fixup_kernel's
 
 template <class T>
 int spmv_dot_impl(const rvvla_crs* A, const T* x, T* y, T* dot, cudaStream_t st) {
@@ -138,25 +187,36 @@ int spmv_dot_impl(const rvvla_crs* A, const T* x, T* y, T* dot, cudaStream_t st)
     return RVVLA_OK;
   }
   const int64_t nw = crs_warp_count(A->nz);
+  const size_t partb = ((size_t)nw * sizeof(T) + 255) / 256 * 256;
+  const size_t sumb = (size_t)dot_blocks(nw) * sizeof(double);
   Scratch sc;
-  RVVLA_CUDA(sc.alloc((size_t)nw * sizeof(T), st));
-  int64_t np = 0;
+  RVVLA_CUDA(sc.alloc(partb + sumb + 256, st));
+  char* base = sc.as<char>();
+  double* out = reinterpret_cast<double*>(base + partb + sumb);
+  CrsDot cd{base, reinterpret_cast<double*>(base + partb), reinterpret_cast<unsigned*>(out + 1), out};
+  RVVLA_CUDA(cudaMemsetAsync(cd.ticket, 0, sizeof(unsigned), st));
   const int rc = std::is_same<T, double>::value
-                     ? crs_spmv_dot_f64(A, reinterpret_cast<const double*>(x), reinterpret_cast<double*>(y),
-                                        sc.as<double>(), nw, &np, st)
-                     : crs_spmv_dot_f32(A, reinterpret_cast<const float*>(x), reinterpret_cast<float*>(y),
-                                        sc.as<float>(), nw, &np, st);
+                     ? crs_spmv_dot_f64(A, reinterpret_cast<const double*>(x), reinterpret_cast<double*>(y), cd, st)
+                     : crs_spmv_dot_f32(A, reinterpret_cast<const float*>(x), reinterpret_cast<float*>(y), cd, st);
   if (rc) return rc;
-  sum_to_kernel<T><<<1, kRedThreads, 0, st>>>(sc.as<T>(), np, dot);
-  RVVLA_LAUNCHED("sum_to_kernel");
+  store_dot_kernel<T><<<1, 1, 0, st>>>(out, dot);
+  RVVLA_LAUNCHED("store_dot_kernel");
   return RVVLA_OK;
 }
 
+// x += alpha p, p = r + beta p: the x update shares the read of p.
 template <class T>
-__global__ void cg_p_kernel(int64_t n, T* __restrict__ p, const T* __restrict__ r, const CgScalars* __restrict__ s) {
-  const T beta = (T)s->beta;
+__global__ void cg_xp_kernel(int64_t n, T* __restrict__ x, T* __restrict__ p, const T* __restrict__ r,
+                             const CgScalars* s, int cur) {
+  grid_chain();
+  const T alpha = (T)cg_alpha(s, cur);
+  const T beta = (T)(s->rr[cur] != 0.0 ? s->rr[cur ^ 1] / s->rr[cur] : 0.0);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = r[i] + beta * p[i];
+  if (i < n) {
+    const T pi = p[i];
+    x[i] += alpha * pi;
+    p[i] = r[i] + beta * pi;
+  }
 }
 
 template <class T>
@@ -174,15 +234,16 @@ int cg_impl(const rvvla_crs* A, const T* b, T* x, int64_t max_iter, double rtol,
   Scratch sc;
   const size_t vec = ((size_t)n * sizeof(T) + 255) / 256 * 256;
   const size_t partb = ((size_t)std::max<int64_t>(nw, 1) * sizeof(T) + 255) / 256 * 256;
+  const size_t sumb = ((size_t)dot_blocks(nw) * sizeof(double) + 255) / 256 * 256;
   const size_t rrb = ((size_t)upd_blocks * sizeof(double) + 255) / 256 * 256;
-  RVVLA_CUDA(sc.alloc(3 * vec + partb + rrb + sizeof(CgScalars), st));
+  RVVLA_CUDA(sc.alloc(3 * vec + partb + sumb + rrb + sizeof(CgScalars), st));
   char* base = sc.as<char>();
   T* r = reinterpret_cast<T*>(base);
   T* p = reinterpret_cast<T*>(base + vec);
   T* q = reinterpret_cast<T*>(base + 2 * vec);
-  T* part = reinterpret_cast<T*>(base + 3 * vec);
-  double* rrp = reinterpret_cast<double*>(base + 3 * vec + partb);
-  CgScalars* s = reinterpret_cast<CgScalars*>(base + 3 * vec + partb + rrb);
+  double* rrp = reinterpret_cast<double*>(base + 3 * vec + partb + sumb);
+  CgScalars* s = reinterpret_cast<CgScalars*>(base + 3 * vec + partb + sumb + rrb);
+  const CrsDot cd{base + 3 * vec, reinterpret_cast<double*>(base + 3 * vec + partb), &s->ticket_dot, &s->pq};
   // r = b - A x, p = r, r.r, b.b
   RVVLA_CUDA(cudaMemcpyAsync(r, b, (size_t)n * sizeof(T), cudaMemcpyDeviceToDevice, st));
   int rc = std::is_same<T, double>::value
@@ -209,31 +270,25 @@ int cg_impl(const rvvla_crs* A, const T* b, T* x, int64_t max_iter, double rtol,
   if ((rc = read_back())) return rc;
   const double bb = hs.bb > 0.0 ? hs.bb : 1.0;
   int64_t it = 0;
-  bool done = std::sqrt(hs.rr / bb) <= rtol;
+  int cur = 0;
+  bool done = std::sqrt(hs.rr[0] / bb) <= rtol;
   while (!done && it < max_iter) {
-    int64_t np = 0;
     rc = std::is_same<T, double>::value
-             ? crs_spmv_dot_f64(A, reinterpret_cast<const double*>(p), reinterpret_cast<double*>(q),
-                                reinterpret_cast<double*>(part), nw, &np, st)
-             : crs_spmv_dot_f32(A, reinterpret_cast<const float*>(p), reinterpret_cast<float*>(q),
-                                reinterpret_cast<float*>(part), nw, &np, st);
+             ? crs_spmv_dot_f64(A, reinterpret_cast<const double*>(p), reinterpret_cast<double*>(q), cd, st)
+             : crs_spmv_dot_f32(A, reinterpret_cast<const float*>(p), reinterpret_cast<float*>(q), cd, st);
     if (rc) return rc;
-    cg_alpha_kernel<T><<<1, kRedThreads, 0, st>>>(part, np, s);
-    RVVLA_LAUNCHED("cg_alpha_kernel");
-    cg_update_kernel<T><<<upd_blocks, kUpdThreads, 0, st>>>(n, x, r, p, q, s, rrp);
-    RVVLA_LAUNCHED("cg_update_kernel");
-    cg_beta_kernel<<<1, kRedThreads, 0, st>>>(rrp, upd_blocks, s);
-    RVVLA_LAUNCHED("cg_beta_kernel");
-    cg_p_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, p, r, s);
-    RVVLA_LAUNCHED("cg_p_kernel");
+    RVVLA_CUDA(launch_chained(cg_update_kernel<T>, (unsigned)upd_blocks, kUpdThreads, st, n, r, q, s, cur, rrp));
+    RVVLA_CUDA(launch_chained(cg_xp_kernel<T>, (unsigned)((n + 255) / 256), 256u, st, n, x, p, r, s, cur));
+    count_launch(2);
+    cur ^= 1;
     ++it;
     if (it % check_every == 0 || it == max_iter) {
       if ((rc = read_back())) return rc;
-      done = std::sqrt(hs.rr / bb) <= rtol;
+      done = std::sqrt(hs.rr[cur] / bb) <= rtol;
     }
   }
   *iters = it;
-  *rel_res = std::sqrt(hs.rr / bb);
+  *rel_res = std::sqrt(hs.rr[cur] / bb);
   return RVVLA_OK;
 }
 
