@@ -14,9 +14,14 @@
 //
 // SpMV: one warp per VHCC thread, lane = vector lane.  Lanes accumulate
 // their products; at an end-of-row vector the warp runs the reference's
-// masked slide-up scan as five __shfl_up steps gated by the stored masks,
-// stores the write lanes' sums to tmp[row_arr[...]] and carries lane 31 into
-// the next vector (:104-140).  Overflow rows are merged into last_row in
+// masked slide-up scan as five __shfl_up steps (the scan masks follow from the
+// write mask, the only one read), stores the write lanes' sums to
+// tmp[row_arr[...]] and carries lane 31 into the next vector (:104-140).  The
+// end-of-row vectors, write masks and rows come from register windows of 32,
+// the next one loaded ahead: reading each where it is needed (masks included,
+// seven dependent loads a vector) took 186 us for the 2M-row power-law matrix
+// in fp32, 135 now (fp64 4M 393 -> 348, fp32 4M 370 -> 263); bound by
+// instructions and the gathers' latency (8 vectors in flight: 156).  Overflow rows are merged into last_row in
 // thread order by a second kernel (the reference's atomic, :157-161), and a
 // third computes y = alpha*tmp + beta*y (:335-397).  Deterministic.
 #include <algorithm>
@@ -145,7 +150,7 @@ __global__ void vhcc_pack_kernel(int64_t total, int64_t nnz, const int* __restri
 // ---------------------------------------------------------------- SpMV
 template <class V, class X, class Ac, class CT>
 __global__ void __launch_bounds__(256)
-vhcc_spmv_kernel(int64_t NT, const int* __restrict__ thr, const uint32_t* __restrict__ veceor,
+vhcc_spmv_kernel(int64_t NT, int n_eor, int n_rows, const int* __restrict__ thr, const uint32_t* __restrict__ veceor,
                  const uint32_t* __restrict__ smask, const uint32_t* __restrict__ row_arr,
                  const uint32_t* __restrict__ col, const V* __restrict__ vals, const X* __restrict__ x,
                  CT* __restrict__ tmp) {
@@ -153,28 +158,50 @@ vhcc_spmv_kernel(int64_t NT, const int* __restrict__ thr, const uint32_t* __rest
   const int lane = threadIdx.x & 31;
   if (t >= NT) return;
   const int* ti = thr + t * 10;
-  int64_t vidx = ti[0], ridx = ti[1];
-  const uint32_t* mk = smask + ((int64_t)ti[2] >> 2);  // sbase is in bytes
-  const int64_t v0 = ti[5], v1 = ti[6];
-  uint32_t eor = veceor[vidx++];
+  const int e0 = ti[0], r0 = ti[1];
+  const uint32_t* mk = smask + ((int64_t)ti[2] >> 2) + kMasks;  // write masks, every (kMasks + 1)th word
+  const int v0 = ti[5], v1 = ti[6];
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
+  // ends of the thread's entries: where the next thread's begin; for the last
+  // thread the arrays' lengths, or, where the descriptor has none, its last
+  // vector (always an end-of-row vector)
+  int ne = 0, nr = 0;
+  if (t + 1 < NT) {
+    ne = ti[10] - e0;
+    nr = ti[11] - r0;
+  } else if (n_eor > 0 && n_rows > 0) {
+    ne = n_eor - 1 - e0;
+    nr = n_rows - r0;
+  } else if (v0 < v1) {
+    do nr += __popc(mk[(int64_t)ne * (kMasks + 1)]);
+    while ((int)veceor[e0 + ne++] < v1 - 1);
+  }
+  // windows of 32 end-of-row vectors (their numbers and write masks) and of 32
+  // rows, lane l holding entry base + l, the next window loaded ahead
+  int ebase = 0, ecur = 0, rbase = 0, rcur = 0;
+  auto ev = [&](int i) { return i < ne ? veceor[e0 + i] : 0xFFFFFFFFu; };
+  auto em = [&](int i) { return i < ne ? mk[(int64_t)i * (kMasks + 1)] : 0u; };
+  auto rw = [&](int i) { return i < nr ? row_arr[r0 + i] : 0u; };
+  uint32_t w_v = ev(lane), w_m = em(lane), w_r = rw(lane);
+  uint32_t n_v = ev(32 + lane), n_m = em(32 + lane), n_r = rw(32 + lane);
+  uint32_t eor = __shfl_sync(0xffffffffu, w_v, 0);
   CT res = 0;
   bool pending = false;  // vectors without a row end left partial sums in every lane
   // vectors kVhccU at a time: all their loads are issued first (indices past
   // the range clamped to its last vector, their products dropped)
-  for (int64_t vb = v0; vb < v1; vb += kVhccU) {
+  for (int vb = v0; vb < v1; vb += kVhccU) {
     uint32_t cc[kVhccU];
     V av[kVhccU];
     X xv[kVhccU];
 #pragma unroll
-    for (int u = 0; u < kVhccU; ++u) cc[u] = ld_stream(col + min(vb + u, v1 - 1) * kVec + lane, pf);
+    for (int u = 0; u < kVhccU; ++u) cc[u] = ld_stream(col + (int64_t)min(vb + u, v1 - 1) * kVec + lane, pf);
 #pragma unroll
-    for (int u = 0; u < kVhccU; ++u) av[u] = ld_stream(vals + min(vb + u, v1 - 1) * kVec + lane, pf);
+    for (int u = 0; u < kVhccU; ++u) av[u] = ld_stream(vals + (int64_t)min(vb + u, v1 - 1) * kVec + lane, pf);
 #pragma unroll
     for (int u = 0; u < kVhccU; ++u) xv[u] = ld_keep(x + cc[u], pl);
 #pragma unroll
     for (int u = 0; u < kVhccU; ++u) {
-      const int64_t v = vb + u;
+      const int v = vb + u;
       if (v >= v1) break;
       const CT prod = (CT)vmul(av[u], xv[u]);
       if ((uint32_t)v != eor) {
@@ -191,21 +218,36 @@ vhcc_spmv_kernel(int64_t NT, const int* __restrict__ thr, const uint32_t* __rest
           pending = false;
         }
         res += prod;
+        const uint32_t wm = __shfl_sync(0xffffffffu, w_m, ecur - ebase);
+        // lanes since the last row end before this one: scan mask s of the
+        // format holds the lanes where that is at least 2^s
+        const uint32_t below = wm & ((1u << lane) - 1u);
+        const int dist = below ? lane - 32 + __clz(below) : lane;
 #pragma unroll
         for (int s = 0; s < kMasks; ++s) {
           const CT o = __shfl_up_sync(0xffffffffu, res, 1 << s);
-          if ((mk[s] >> lane) & 1u) res += o;
+          if (dist >= (1 << s)) res += o;
         }
-        const uint32_t wm = mk[kMasks];
-        if ((wm >> lane) & 1u) {
-          const int rank = __popc(wm & ((1u << lane) - 1u));
-          tmp[row_arr[ridx + rank]] = res;
+        // the vector's rows: at most 32, so in this window or the next
+        const int rank = rcur - rbase + __popc(below);
+        const uint32_t ra = __shfl_sync(0xffffffffu, w_r, rank & 31), rb = __shfl_sync(0xffffffffu, n_r, rank & 31);
+        if ((wm >> lane) & 1u) tmp[rank < 32 ? ra : rb] = res;
+        rcur += __popc(wm);
+        if (rcur - rbase >= 32) {
+          rbase += 32;
+          w_r = n_r;
+          n_r = rw(rbase + 32 + lane);
         }
-        ridx += __popc(wm);
         const CT carry = ((wm >> 31) & 1u) ? CT(0) : __shfl_sync(0xffffffffu, res, 31);
         res = (lane == 0) ? carry : CT(0);
-        mk += kMasks + 1;
-        eor = veceor[vidx++];
+        if (++ecur - ebase == 32) {
+          ebase += 32;
+          w_v = n_v;
+          w_m = n_m;
+          n_v = ev(ebase + 32 + lane);
+          n_m = em(ebase + 32 + lane);
+        }
+        eor = __shfl_sync(0xffffffffu, w_v, ecur - ebase);
       }
     }
   }
@@ -253,7 +295,7 @@ int vhcc_spmv_impl(const rvvla_vhcc* A, X alpha, const X* x, X beta, X* y, cudaS
   RVVLA_CUDA(cudaMemsetAsync(tmp, 0, (size_t)A->pad_rows * sizeof(CT), st));
   const int64_t NT = A->num_threads;
   vhcc_spmv_kernel<V, X, Ac, CT><<<(unsigned)((NT * 32 + 255) / 256), 256, 0, st>>>(
-      NT, A->thr_info, A->veceor_ptr, (const uint32_t*)A->scan_mask, A->row_arr, A->col_arr, (const V*)A->vals_arr, x,
+      NT, (int)A->n_eor, (int)A->n_rowarr, A->thr_info, A->veceor_ptr, (const uint32_t*)A->scan_mask, A->row_arr, A->col_arr, (const V*)A->vals_arr, x,
       tmp);
   RVVLA_LAUNCHED("vhcc_spmv_kernel");
   vhcc_overflow_kernel<CT><<<(unsigned)((NT + 255) / 256), 256, 0, st>>>(NT, A->num_rows, A->thr_info, tmp);
