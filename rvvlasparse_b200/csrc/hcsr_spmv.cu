@@ -519,7 +519,7 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
   using P = typename Ty::P;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_w[3 * kHW];
-  const HLayout<SA, P> L(GACC ? 0 : R);
+  const HLayout<SA, P> L(GACC ? 0 : min(R, m));  // as the launch sizes it
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t br = blockIdx.x;
   const int64_t r0 = br * R;
