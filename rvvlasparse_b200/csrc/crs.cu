@@ -99,6 +99,7 @@ __global__ void crs_compact_kernel(int m, int nnz, const int* __restrict__ Rst, 
 
 template <class X>
 __global__ void crs_empty_rows_kernel(int me, const int* __restrict__ empty, X* __restrict__ y, X beta) {
+  chain_open();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < me) {
     const int r = empty[i];
@@ -244,49 +245,31 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
     CT* cval = (CT*)(sc.as<char>() + row_bytes);
     const unsigned blocks = (unsigned)((nw * 32 + 255) / 256);
     CT* dot_part = dot ? reinterpret_cast<CT*>(dot->part) : nullptr;
-    if (dot_part) {
-      const bool vec = (uintptr_t)A->Col % 16 == 0 && (uintptr_t)A->Val % 16 == 0;
-      auto kern = vec ? crs_run_kernel<V, X, Ac, CT, true, false, true> : crs_run_kernel<V, X, Ac, CT, false, false, true>;
-      RVVLA_CUDA(launch_chained(kern, blocks, 256, st, mr, (int)A->nz, E, (int)nw, rst, bits, A->Col,
-                                (const V*)A->Val, x, y, alpha, beta, wrow, crow, cval, row_map, nullptr, dot_part));
-      count_launch();
-    } else if (perm) {
-      const bool vec = (uintptr_t)A->Col % 16 == 0 && (uintptr_t)perm % 16 == 0;
-      if (vec)
-        crs_run_kernel<V, X, Ac, CT, true, true><<<blocks, 256, 0, st>>>(
-            mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, pval, x, y, alpha, beta, wrow, crow, cval, row_map,
-            perm);
-      else
-        crs_run_kernel<V, X, Ac, CT, false, true><<<blocks, 256, 0, st>>>(
-            mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, pval, x, y, alpha, beta, wrow, crow, cval, row_map,
-            perm);
-      RVVLA_LAUNCHED("crs_run_kernel");
-    } else if (crs_use_stream_kernel()) {
-      crs_stream_kernel<V, X, Ac, CT><<<blocks, 256, 0, st>>>(mr, (int)A->nz, E, (int)nw, rst, A->Col,
-                                                              (const V*)A->Val, x, y, alpha, beta, wrow, crow, cval,
-                                                              row_map);
+    const V* val = perm ? pval : (const V*)A->Val;
+    // 16-byte loads where Col and the values or their permutation allow them
+    const bool vec = (uintptr_t)A->Col % 16 == 0 && (uintptr_t)(perm ? (const void*)perm : (const void*)val) % 16 == 0;
+    // the solvers' products follow kernels of the same call, the others at
+    // most the empty rows'
+    const bool chained = dot != nullptr || mr < (int)A->m;
+    if (!dot && !perm && crs_use_stream_kernel()) {
+      crs_stream_kernel<V, X, Ac, CT><<<blocks, 256, 0, st>>>(mr, (int)A->nz, E, (int)nw, rst, A->Col, val, x, y, alpha,
+                                                              beta, wrow, crow, cval, row_map);
       RVVLA_LAUNCHED("crs_stream_kernel");
     } else {
-      const bool vec = (uintptr_t)A->Col % 16 == 0 && (uintptr_t)A->Val % 16 == 0;
-      if (vec)
-        crs_run_kernel<V, X, Ac, CT, true><<<blocks, 256, 0, st>>>(mr, (int)A->nz, E, (int)nw, rst, bits,
-                                                                   A->Col, (const V*)A->Val, x, y, alpha, beta, wrow,
-                                                                   crow, cval, row_map);
-      else
-        crs_run_kernel<V, X, Ac, CT, false><<<blocks, 256, 0, st>>>(mr, (int)A->nz, E, (int)nw, rst, bits,
-                                                                    A->Col, (const V*)A->Val, x, y, alpha, beta, wrow,
-                                                                    crow, cval, row_map);
-      RVVLA_LAUNCHED("crs_run_kernel");
+      auto kern = dot    ? (vec ? crs_run_kernel<V, X, Ac, CT, true, false, true>
+                                : crs_run_kernel<V, X, Ac, CT, false, false, true>)
+                  : perm ? (vec ? crs_run_kernel<V, X, Ac, CT, true, true> : crs_run_kernel<V, X, Ac, CT, false, true>)
+                         : (vec ? crs_run_kernel<V, X, Ac, CT, true> : crs_run_kernel<V, X, Ac, CT, false>);
+      RVVLA_CHAIN(chained, kern, blocks, 256, st, mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, val, x, y, alpha, beta,
+                  wrow, crow, cval, row_map, perm, dot_part);
     }
     const unsigned fix_blocks = (unsigned)((2 * nw + 255) / 256);
-    if (dot) {
-      RVVLA_CUDA(launch_chained(crs_dot_fixup_kernel<X, CT>, fix_blocks, 256, st, (int)nw, crow, cval, y, alpha, beta,
-                                row_map, dot_part, dot->sums, dot->ticket, dot->out));
-      count_launch();
-    } else {
-      crs_stream_fixup_kernel<X, CT><<<fix_blocks, 256, 0, st>>>((int)(2 * nw), crow, cval, y, alpha, beta, row_map);
-      RVVLA_LAUNCHED("crs_stream_fixup_kernel");
-    }
+    if (dot)
+      RVVLA_CHAIN(true, (crs_dot_fixup_kernel<X, CT>), fix_blocks, 256, st, (int)nw, crow, cval, y, alpha, beta, row_map,
+                  dot_part, dot->sums, dot->ticket, dot->out);
+    else
+      RVVLA_CHAIN(true, (crs_stream_fixup_kernel<X, CT>), fix_blocks, 256, st, (int)(2 * nw), crow, cval, y, alpha, beta,
+                  row_map);
     return RVVLA_OK;
   }
   const int64_t nt = crs_tiles(A->m, A->nz, IPT);

@@ -102,7 +102,7 @@ crs_run_kernel(int m, int nnz, int E, int nwarps, const int* __restrict__ rst, c
                CT* __restrict__ dot_part = nullptr) {
   const int w = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  if constexpr (DOT) grid_chain();  // the solvers chain their kernels
+  grid_chain();
   if (w >= nwarps) return;
   const int kb = w * E;
   const int ke = min(nnz, kb + E);

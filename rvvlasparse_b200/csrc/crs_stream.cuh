@@ -194,6 +194,7 @@ template <class X, class CT>
 __global__ void crs_stream_fixup_kernel(int nslots, const int* __restrict__ carry_row,
                                         const CT* __restrict__ carry_val, X* __restrict__ y, X alpha, X beta,
                                         const int* __restrict__ row_map) {
+  grid_chain();
   crs_fixup_slot((int)(blockIdx.x * blockDim.x + threadIdx.x), nslots, carry_row, carry_val, y, alpha, beta, row_map);
 }
 

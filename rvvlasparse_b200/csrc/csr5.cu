@@ -260,6 +260,7 @@ csr5_spmv_kernel(int64_t nfull, int tiles_per_warp, const uint32_t* __restrict__
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kC5Warps * S * Cfg::STAGE_B) + wid * S;
   const int64_t warp = (int64_t)blockIdx.x * kC5Warps + wid;
   const int64_t t0 = warp * tiles_per_warp;
+  chain_open();
   if (t0 >= nfull) return;
   const int64_t t1 = min(nfull, t0 + tiles_per_warp);
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -462,6 +463,7 @@ csr5_spmv_generic_kernel(int64_t nfull, int tiles_per_warp, int sigma, int by, i
   const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int64_t t0 = warp * tiles_per_warp;
+  chain_open();
   if (t0 >= nfull) return;
   const int64_t t1 = min(nfull, t0 + tiles_per_warp);
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
@@ -581,6 +583,7 @@ csr5_spmv_generic_kernel(int64_t nfull, int tiles_per_warp, int sigma, int by, i
 template <class X, class CT>
 __global__ void csr5_calibrate_kernel(int64_t nwarps, const int* __restrict__ cal_row, const CT* __restrict__ cal,
                                       X* __restrict__ y, X alpha) {
+  grid_chain();
   const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nwarps) return;
   const int r = cal_row[w];
@@ -599,6 +602,7 @@ __global__ void csr5_tail_kernel(int64_t m, int64_t tail_row, int64_t tail_start
                                  const uint32_t* __restrict__ colidx, const V* __restrict__ vals,
                                  const X* __restrict__ x, X* __restrict__ y, X alpha, X beta) {
   using Ops = LaneOps<V, X, Ac, CT>;
+  grid_chain();
   const int64_t r = tail_row + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= m) return;
@@ -618,6 +622,7 @@ __global__ void csr5_tail_kernel(int64_t m, int64_t tail_row, int64_t tail_start
 
 template <class X>
 __global__ void scale_kernel(int64_t m, X* __restrict__ y, X beta) {
+  chain_open();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) y[i] = (beta == X(0)) ? X(0) : beta * y[i];
 }
@@ -764,15 +769,13 @@ int csr5_spmv_impl(const rvvla_csr5* A, X alpha, const X* x, X beta, X* y, cudaS
             A->tile_pointer, A->tile_descriptor, eo_ptr, eo, x, y, alpha, beta_eff, cal, cal_row);
     }
     RVVLA_LAUNCHED("csr5_spmv_kernel");
-    csr5_calibrate_kernel<X, CT><<<(unsigned)((nwarps + 255) / 256), 256, 0, st>>>(nwarps, cal_row, cal, y, alpha);
-    RVVLA_LAUNCHED("csr5_calibrate_kernel");
+    RVVLA_CHAIN(true, (csr5_calibrate_kernel<X, CT>), (nwarps + 255) / 256, 256, st, nwarps, cal_row, cal, y, alpha);
   }
   if (A->tail_tile_start < A->m) {
     const int64_t rows = A->m - A->tail_tile_start;
-    csr5_tail_kernel<V, X, Ac, CT><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(
-        A->m, A->tail_tile_start, (int64_t)(A->p - 1) * A->omega * A->sigma, A->csr_row_pointer, A->csr_column_index,
-        (const V*)A->csr_value, x, y, alpha, beta_eff);
-    RVVLA_LAUNCHED("csr5_tail_kernel");
+    RVVLA_CHAIN(nfull > 0 || !A->no_empty_rows, (csr5_tail_kernel<V, X, Ac, CT>), (rows + 7) / 8, 256, st, A->m,
+                A->tail_tile_start, (int64_t)(A->p - 1) * A->omega * A->sigma, A->csr_row_pointer, A->csr_column_index,
+                (const V*)A->csr_value, x, y, alpha, beta_eff);
   }
   return RVVLA_OK;
 }

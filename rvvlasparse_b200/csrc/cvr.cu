@@ -165,6 +165,7 @@ __global__ void cvr_empty_kernel(int64_t m, const int* __restrict__ Rst, int* __
 // ---------------------------------------------------------------- SpMV
 template <class X>
 __global__ void cvr_scale_kernel(int64_t m, X* __restrict__ y, X beta) {
+  chain_open();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) y[i] = (beta == X(0)) ? X(0) : y[i] * beta;
 }
@@ -295,6 +296,7 @@ cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ 
     }
     __syncwarp();
   };
+  chain_wait();  // y is scaled
   int64_t v = vb;
   for (; v < ve; v += kCvrU) {
     uint32_t c[kCvrU];
@@ -368,10 +370,8 @@ int cvr_spmv_impl(const rvvla_cvr* A, X alpha, const X* x, X beta, X* y, cudaStr
   RVVLA_LAUNCHED("cvr_scale_kernel");
   const int64_t NT = A->Nthreads_avail;
   const int64_t nrec = (A->n_record - 2) / 2;
-  cvr_spmv_kernel<V, X, CT><<<(unsigned)((NT * kCvrSplit + 7) / 8), 256, 0, st>>>(
-      NT, A->nItems, nrec, (const V*)A->vPack_vec_vals, A->vPack_vec_cols, A->vPack_vec_record,
-      A->writeback_pos_record, x, y, alpha);
-  RVVLA_LAUNCHED("cvr_spmv_kernel");
+  RVVLA_CHAIN(true, (cvr_spmv_kernel<V, X, CT>), (NT * kCvrSplit + 7) / 8, 256, st, NT, A->nItems, nrec,
+              (const V*)A->vPack_vec_vals, A->vPack_vec_cols, A->vPack_vec_record, A->writeback_pos_record, x, y, alpha);
   return RVVLA_OK;
 }
 

@@ -118,6 +118,9 @@ lav_fused_kernel(int64_t nseg, int64_t cc, int64_t m, int64_t n, int64_t nlong, 
   static_assert(32 % L == 0, "a chunk must not straddle warps");
   constexpr int G = 256 / L;
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
+  chain_open();
+  // (the sums run while the sparse part's kernels drain; y is touched after
+  // chain_wait)
   const int64_t nmax = n > 0 ? n - 1 : 0;
   if ((int64_t)blockIdx.x < nlong) {
     __shared__ CT red[256];
@@ -140,6 +143,7 @@ lav_fused_kernel(int64_t nseg, int64_t cc, int64_t m, int64_t n, int64_t nlong, 
       __syncthreads();
     }
     const int64_t gs = c * L + threadIdx.x;
+    chain_wait();
     if (threadIdx.x < L && gs < m) {
       const uint32_t r = row_order[gs];
       y[r] += alpha * (X)acc;
@@ -166,6 +170,7 @@ lav_fused_kernel(int64_t nseg, int64_t cc, int64_t m, int64_t n, int64_t nlong, 
     acc += __shfl_sync(0xffffffffu, part, (lane & ~(L - 1)) + src);
   }
   const int64_t g = c * L + i;
+  chain_wait();
   if (live && g < m) {
     const uint32_t r = row_order[g];
     y[r] += alpha * (X)acc;
@@ -228,12 +233,9 @@ int lav_spmv_impl(const rvvla_lav* A, X alpha, const X* x, X beta, X* y, cudaStr
     switch (A->SIMD_Lanes) {
 #define LAV_FUSED(LN)                                                                                          \
   case LN:                                                                                                     \
-    lav_fused_kernel<V, X, CT, LN><<<blocks, 256, 0, st>>>(A->segment_count, A->chunk_count, A->m, A->n,       \
-                                                          nlong,                                              \
-                                                          A->chunk_offsets, A->chunk_offsets_full_mask,       \
-                                                          A->segment_ptr, A->mask, (const V*)A->val,          \
-                                                          A->col_id, A->lane_of_slot, A->row_order, x, y,     \
-                                                          alpha);                                             \
+    RVVLA_CHAIN(true, (lav_fused_kernel<V, X, CT, LN>), blocks, 256, st, A->segment_count, A->chunk_count, A->m, \
+                A->n, nlong, A->chunk_offsets, A->chunk_offsets_full_mask, A->segment_ptr, A->mask,            \
+                (const V*)A->val, A->col_id, A->lane_of_slot, A->row_order, x, y, alpha);                      \
     break;
       LAV_FUSED(1)
       LAV_FUSED(2)
@@ -243,7 +245,6 @@ int lav_spmv_impl(const rvvla_lav* A, X alpha, const X* x, X beta, X* y, cudaStr
       LAV_FUSED(32)
 #undef LAV_FUSED
     }
-    RVVLA_LAUNCHED("lav_fused_kernel");
     return RVVLA_OK;
   }
   for (int64_t s = 0; s < A->segment_count; ++s) {

@@ -54,6 +54,13 @@ inline void prefer_shared(K kernel) {
 // it could not be made.
 cudaMemPool_t scratch_pool();
 
+// A launch chained to the stream's previous kernel if `chained`.
+#define RVVLA_CHAIN(chained, kernel, blocks, threads, st, ...)                                        \
+  do {                                                                                                \
+    RVVLA_CUDA(::rvvla::launch_chained(kernel, (unsigned)(blocks), threads, chained, st, __VA_ARGS__)); \
+    ::rvvla::count_launch();                                                                          \
+  } while (0)
+
 // Stream-ordered temporary buffer.  It comes from the library's own pool,
 // which keeps up to kScratchKeep bytes when a stream is synchronised: the
 // device's default pool keeps none, so the first product after a
@@ -94,13 +101,16 @@ struct CrsDot {
 };
 
 // Launches that may start while the stream's previous kernel drains: the
-// kernel calls grid_chain() before it touches anything that kernel writes or
-// reads.  In a chain of short kernels this hides the launch and the ramp-up.
+// kernel calls grid_chain() (or chain_wait() later) before it touches anything
+// the kernels before it write or read.  In a chain of short kernels this hides
+// launches and ramp-ups.  The first kernel of a call is launched the ordinary
+// way, so that whatever the caller enqueued before is complete.
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t st, A... args) {
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned blocks, unsigned threads, bool chained, cudaStream_t st,
+                                  A... args) {
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = chained ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
@@ -110,13 +120,15 @@ inline cudaError_t launch_chained(void (*kernel)(P...), unsigned blocks, unsigne
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// By every CTA that does any work: lets the stream's next chained kernel start
-// once all CTAs have come here, and waits until the previous kernel is
-// complete and its writes are visible.  Neither does anything in a kernel
-// launched the ordinary way.
+// By every CTA that does any work: chain_open lets the stream's next chained
+// kernel start once all CTAs have come here, chain_wait waits until the
+// previous kernel is complete and its writes are visible (at once in a kernel
+// launched the ordinary way).
+__device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_chain() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  chain_open();
+  chain_wait();
 }
 
 // ------------------------------------------------------------------ loads

@@ -277,9 +277,8 @@ int cg_impl(const rvvla_crs* A, const T* b, T* x, int64_t max_iter, double rtol,
              ? crs_spmv_dot_f64(A, reinterpret_cast<const double*>(p), reinterpret_cast<double*>(q), cd, st)
              : crs_spmv_dot_f32(A, reinterpret_cast<const float*>(p), reinterpret_cast<float*>(q), cd, st);
     if (rc) return rc;
-    RVVLA_CUDA(launch_chained(cg_update_kernel<T>, (unsigned)upd_blocks, kUpdThreads, st, n, r, q, s, cur, rrp));
-    RVVLA_CUDA(launch_chained(cg_xp_kernel<T>, (unsigned)((n + 255) / 256), 256u, st, n, x, p, r, s, cur));
-    count_launch(2);
+    RVVLA_CHAIN(true, cg_update_kernel<T>, upd_blocks, kUpdThreads, st, n, r, q, s, cur, rrp);
+    RVVLA_CHAIN(true, cg_xp_kernel<T>, (n + 255) / 256, 256, st, n, x, p, r, s, cur);
     cur ^= 1;
     ++it;
     if (it % check_every == 0 || it == max_iter) {

@@ -156,6 +156,7 @@ vhcc_spmv_kernel(int64_t NT, int n_eor, int n_rows, const int* __restrict__ thr,
                  CT* __restrict__ tmp) {
   const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  chain_open();
   if (t >= NT) return;
   const int* ti = thr + t * 10;
   const int e0 = ti[0], r0 = ti[1];
@@ -256,6 +257,7 @@ vhcc_spmv_kernel(int64_t NT, int n_eor, int n_rows, const int* __restrict__ thr,
 // overflow rows into last_row, in thread order (the reference's atomic add)
 template <class CT>
 __global__ void vhcc_overflow_kernel(int64_t NT, int64_t m, const int* __restrict__ thr, CT* __restrict__ tmp) {
+  grid_chain();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= NT) return;
   const int r = thr[t * 10 + 3];
@@ -268,6 +270,7 @@ __global__ void vhcc_overflow_kernel(int64_t NT, int64_t m, const int* __restric
 
 template <class X, class CT>
 __global__ void vhcc_out_kernel(int64_t m, const CT* __restrict__ tmp, X* __restrict__ y, X alpha, X beta) {
+  grid_chain();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) write_row(y, (int)i, alpha, beta, (X)tmp[i]);
 }
@@ -298,10 +301,8 @@ int vhcc_spmv_impl(const rvvla_vhcc* A, X alpha, const X* x, X beta, X* y, cudaS
       NT, (int)A->n_eor, (int)A->n_rowarr, A->thr_info, A->veceor_ptr, (const uint32_t*)A->scan_mask, A->row_arr, A->col_arr, (const V*)A->vals_arr, x,
       tmp);
   RVVLA_LAUNCHED("vhcc_spmv_kernel");
-  vhcc_overflow_kernel<CT><<<(unsigned)((NT + 255) / 256), 256, 0, st>>>(NT, A->num_rows, A->thr_info, tmp);
-  RVVLA_LAUNCHED("vhcc_overflow_kernel");
-  vhcc_out_kernel<X, CT><<<(unsigned)((A->num_rows + 255) / 256), 256, 0, st>>>(A->num_rows, tmp, y, alpha, beta);
-  RVVLA_LAUNCHED("vhcc_out_kernel");
+  RVVLA_CHAIN(true, vhcc_overflow_kernel<CT>, (NT + 255) / 256, 256, st, NT, A->num_rows, A->thr_info, tmp);
+  RVVLA_CHAIN(true, (vhcc_out_kernel<X, CT>), (A->num_rows + 255) / 256, 256, st, A->num_rows, tmp, y, alpha, beta);
   return RVVLA_OK;
 }
 
