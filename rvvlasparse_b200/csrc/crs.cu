@@ -39,6 +39,7 @@
 
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 
 namespace rvvla {
 
@@ -54,8 +55,9 @@ __global__ void crs_run_bits_kernel(int m, const int* __restrict__ rst, uint32_t
 // SMs x 32 resident warps), so a medium-size matrix does not leave a large
 // partial last wave.  A function of nz alone: the analysis and the SpMV
 // agree on it.
+constexpr int kRunSpanMax = 2048;
 int crs_warp_span(int64_t nz) {
-  int E = 2048;
+  int E = kRunSpanMax;
   while (E > 256 && nz < (int64_t)6 * 4736 * E) E >>= 1;
   return E;
 }
@@ -256,12 +258,27 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
                                                               beta, wrow, crow, cval, row_map);
       RVVLA_LAUNCHED("crs_stream_kernel");
     } else {
-      auto kern = dot    ? (vec ? crs_run_kernel<V, X, Ac, CT, true, false, true>
-                                : crs_run_kernel<V, X, Ac, CT, false, false, true>)
-                  : perm ? (vec ? crs_run_kernel<V, X, Ac, CT, true, true> : crs_run_kernel<V, X, Ac, CT, false, true>)
-                         : (vec ? crs_run_kernel<V, X, Ac, CT, true> : crs_run_kernel<V, X, Ac, CT, false>);
-      RVVLA_CHAIN(chained, kern, blocks, 256, st, mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, val, x, y, alpha, beta,
-                  wrow, crow, cval, row_map, perm, dot_part);
+      // CTAs of 4 warps, whose slots turn over sooner and whose registers round
+      // to one warp per scheduler more (random rows n = 10^6 mean 8 fp64 57.5 ->
+      // 55.4 us with 4 warps instead of 8, mean 19 110 -> 105, Laplacian 2048^2
+      // fp64 82 -> 75, stencil 128^3 183 -> 174), but of 8 at the longest span,
+      // where a warp's rows spread far enough that neighbouring warps sharing
+      // L1 count for more (power law 4M fp64: 278 us with 4, 259 with 8, 270
+      // with 32).  Registers capped for 40 or 48 warps per SM: 81 and 85 us on
+      // the Laplacian.
+      auto run = [&](auto tpb) -> int {
+        constexpr int T = decltype(tpb)::value;
+        auto kern = dot    ? (vec ? crs_run_kernel<V, X, Ac, CT, T, true, false, true>
+                                  : crs_run_kernel<V, X, Ac, CT, T, false, false, true>)
+                    : perm ? (vec ? crs_run_kernel<V, X, Ac, CT, T, true, true>
+                                  : crs_run_kernel<V, X, Ac, CT, T, false, true>)
+                           : (vec ? crs_run_kernel<V, X, Ac, CT, T, true> : crs_run_kernel<V, X, Ac, CT, T, false>);
+        RVVLA_CHAIN(chained, kern, (nw * 32 + T - 1) / T, T, st, mr, (int)A->nz, E, (int)nw, rst, bits, A->Col, val, x,
+                    y, alpha, beta, wrow, crow, cval, row_map, perm, dot_part);
+        return RVVLA_OK;
+      };
+      rc = E >= kRunSpanMax ? run(std::integral_constant<int, 256>()) : run(std::integral_constant<int, 128>());
+      if (rc) return rc;
     }
     const unsigned fix_blocks = (unsigned)((2 * nw + 255) / 256);
     if (dot)

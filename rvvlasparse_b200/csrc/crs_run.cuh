@@ -93,8 +93,9 @@ __device__ __forceinline__ void run_idx(const int* p, int (&v)[kRunLane], uint64
 // also adds x[row] * v to the warp's partial dot_part[w], so the warps'
 // partials sum to x^T (A x) without a second pass over y (the solvers'
 // fused SpMV-dot; square A).
-template <class V, class X, class Ac, class CT, bool VEC, bool PERM = false, bool DOT = false>
-__global__ void __launch_bounds__(256)
+// TPB: threads per CTA (the warps do not cooperate).
+template <class V, class X, class Ac, class CT, int TPB, bool VEC, bool PERM = false, bool DOT = false>
+__global__ void __launch_bounds__(TPB)
 crs_run_kernel(int m, int nnz, int E, int nwarps, const int* __restrict__ rst, const uint32_t* __restrict__ bits,
                const int* __restrict__ Col, const V* __restrict__ Val, const X* __restrict__ x, X* __restrict__ y,
                X alpha, X beta, const int* __restrict__ wrow, int* __restrict__ carry_row, CT* __restrict__ carry_val,
