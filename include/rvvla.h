@@ -27,9 +27,10 @@
  *   - Descriptor structs mirror the reference classes' public fields (same
  *     names, same meaning), with device pointers.
  *   - Entry points that need temporary device memory obtain it stream-ordered
- *     on `stream`, from a memory pool of the library's own (the ordinary fp64
- *     CSR5 entry: from the device's default pool).  Between calls that pool
- *     keeps at most 256 MB per device; rvvla_trim_scratch() gives it back.
+ *     on `stream`: products and solvers from a memory pool of the library's own
+ *     (the ordinary fp64 CSR5 product, requests above 256 MB and the builders:
+ *     from the device's default pool).  Between calls that pool keeps at most
+ *     256 MB per device; rvvla_trim_scratch() gives it back.
  */
 #ifndef RVVLA_H
 #define RVVLA_H

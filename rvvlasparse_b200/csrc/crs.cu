@@ -242,7 +242,7 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
     }
     Scratch sc;
     const size_t row_bytes = ((size_t)(2 * nw) * sizeof(int32_t) + 255) / 256 * 256;
-    RVVLA_CUDA(sc.alloc(row_bytes + (size_t)(2 * nw) * sizeof(CT), st));
+    RVVLA_CUDA(sc.alloc_kept(row_bytes + (size_t)(2 * nw) * sizeof(CT), st));
     int32_t* crow = sc.as<int32_t>();
     CT* cval = (CT*)(sc.as<char>() + row_bytes);
     const unsigned blocks = (unsigned)((nw * 32 + 255) / 256);
@@ -297,7 +297,7 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
   const size_t row_off = (plan_bytes + 255) / 256 * 256;
   const size_t val_off = row_off + ((size_t)nt * sizeof(int32_t) + 255) / 256 * 256;
   Scratch sc;
-  RVVLA_CUDA(sc.alloc(val_off + (size_t)nt * sizeof(CT), st));
+  RVVLA_CUDA(sc.alloc_kept(val_off + (size_t)nt * sizeof(CT), st));
   char* base = sc.as<char>();
   if (!plan) {
     rc = crs_plan_launch(A->m, A->nz, A->Rst, IPT, (int32_t*)base, st);

@@ -729,7 +729,7 @@ int csr5_spmv_impl(const rvvla_csr5* A, X alpha, const X* x, X beta, X* y, cudaS
     int* cal_row = cal_row_buf;
     if (!cal) {
       const size_t cal_bytes = (size_t)nwarps * (sizeof(CT) + sizeof(int)) + 256;
-      RVVLA_CUDA(sizeof(V) == 8 ? sc.alloc_default(cal_bytes, st) : sc.alloc(cal_bytes, st));
+      RVVLA_CUDA(sizeof(V) == 8 ? sc.alloc(cal_bytes, st) : sc.alloc_kept(cal_bytes, st));
       cal = sc.as<CT>();
       cal_row = reinterpret_cast<int*>(sc.as<char>() + ((size_t)nwarps * sizeof(CT) + 255) / 256 * 256);
     } else if (nwarps > cal_cap) {

@@ -838,7 +838,7 @@ int hcsr_spmv_impl(const rvvla_hcsr* A, X alpha, const X* x, X beta, X* y, cudaS
   // block rows too tall for shared memory: the accumulator is a global
   // scratch array (each CTA owns its slice)
   Scratch sc;
-  RVVLA_CUDA(sc.alloc((size_t)A->m * sizeof(SA), st));
+  RVVLA_CUDA(sc.alloc_kept((size_t)A->m * sizeof(SA), st));
   const size_t smem_g = HLayout<SA, P>(0).total;
   return vec ? hcsr_launch<V, X, SA, MIX, true, true>(A, alpha, x, beta, y, sc.as<SA>(), smem_g, st)
              : hcsr_launch<V, X, SA, MIX, false, true>(A, alpha, x, beta, y, sc.as<SA>(), smem_g, st);

@@ -61,27 +61,29 @@ cudaMemPool_t scratch_pool();
     ::rvvla::count_launch();                                                                          \
   } while (0)
 
-// Stream-ordered temporary buffer.  It comes from the library's own pool,
-// which keeps up to kScratchKeep bytes when a stream is synchronised: the
-// device's default pool keeps none, so the first product after a
+// Stream-ordered temporary buffer.  alloc() takes it from the device's default
+// pool (builders, and the ordinary fp64 CSR5 product, whose callers account
+// for that pool).  alloc_kept() is for products: it takes up to kScratchKeep
+// bytes from the library's own pool, which keeps that much when a stream is
+// synchronised; the default pool keeps nothing, so the first product after a
 // synchronisation mapped its few KB of carries anew (the CRS fp64 product of
-// 4M power-law rows, first call on a new matrix: 883 us, 406 us with this
-// pool).  Larger buffers (builders) come from the default pool as before.
+// 4M power-law rows, first call on a new matrix: 883 us, 406 us with the kept
+// pool; a first CG solve on 4M rows 8.7 -> 6.0 ms).  Builders stay away from
+// it: the LAV builder's buffers, trimmed to the limit at each of its
+// synchronisations, took 118 ms instead of 31.
 constexpr uint64_t kScratchKeep = 256ull << 20;  // a solve on 8M rows in fp64 fits
 struct Scratch {
   void* p = nullptr;
   cudaStream_t s = nullptr;
   cudaError_t alloc(size_t bytes, cudaStream_t st) {
     s = st;
-    if (bytes == 0) bytes = 16;
-    cudaMemPool_t pool = bytes <= kScratchKeep ? scratch_pool() : nullptr;
-    return pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMallocAsync(&p, bytes, st);
-  }
-  // From the device's default pool, as callers that account for that pool
-  // expect of the ordinary fp64 CSR5 entry.
-  cudaError_t alloc_default(size_t bytes, cudaStream_t st) {
-    s = st;
     return cudaMallocAsync(&p, bytes == 0 ? 16 : bytes, st);
+  }
+  cudaError_t alloc_kept(size_t bytes, cudaStream_t st) {
+    cudaMemPool_t pool = bytes <= kScratchKeep ? scratch_pool() : nullptr;
+    if (!pool) return alloc(bytes, st);
+    s = st;
+    return cudaMallocFromPoolAsync(&p, bytes == 0 ? 16 : bytes, pool, st);
   }
   ~Scratch() {
     if (p) cudaFreeAsync(p, s);

@@ -238,7 +238,7 @@ int sell_spmv_impl(const rvvla_sell* A, int stage, X alpha, const X* x, X beta, 
   const unsigned blocks = (unsigned)((A->m + 255) / 256);
   if (stage == RVVLA_STAGE_PREPARATION || stage == RVVLA_STAGE_GET_RESULTS) {
     Scratch sc;
-    RVVLA_CUDA(sc.alloc((size_t)A->m * sizeof(X), st));
+    RVVLA_CUDA(sc.alloc_kept((size_t)A->m * sizeof(X), st));
     RVVLA_CUDA(cudaMemcpyAsync(sc.p, y, (size_t)A->m * sizeof(X), cudaMemcpyDeviceToDevice, st));
     sell_permute_kernel<X><<<blocks, 256, 0, st>>>(A->m, A->vPerm, sc.as<X>(), y,
                                                    stage == RVVLA_STAGE_PREPARATION ? 1 : 0);

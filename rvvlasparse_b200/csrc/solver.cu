@@ -190,7 +190,7 @@ int spmv_dot_impl(const rvvla_crs* A, const T* x, T* y, T* dot, cudaStream_t st)
   const size_t partb = ((size_t)nw * sizeof(T) + 255) / 256 * 256;
   const size_t sumb = (size_t)dot_blocks(nw) * sizeof(double);
   Scratch sc;
-  RVVLA_CUDA(sc.alloc(partb + sumb + 256, st));
+  RVVLA_CUDA(sc.alloc_kept(partb + sumb + 256, st));
   char* base = sc.as<char>();
   double* out = reinterpret_cast<double*>(base + partb + sumb);
   CrsDot cd{base, reinterpret_cast<double*>(base + partb), reinterpret_cast<unsigned*>(out + 1), out};
@@ -236,7 +236,7 @@ int cg_impl(const rvvla_crs* A, const T* b, T* x, int64_t max_iter, double rtol,
   const size_t partb = ((size_t)std::max<int64_t>(nw, 1) * sizeof(T) + 255) / 256 * 256;
   const size_t sumb = ((size_t)dot_blocks(nw) * sizeof(double) + 255) / 256 * 256;
   const size_t rrb = ((size_t)upd_blocks * sizeof(double) + 255) / 256 * 256;
-  RVVLA_CUDA(sc.alloc(3 * vec + partb + sumb + rrb + sizeof(CgScalars), st));
+  RVVLA_CUDA(sc.alloc_kept(3 * vec + partb + sumb + rrb + sizeof(CgScalars), st));
   char* base = sc.as<char>();
   T* r = reinterpret_cast<T*>(base);
   T* p = reinterpret_cast<T*>(base + vec);
@@ -421,7 +421,7 @@ int bicgstab_impl(const rvvla_crs* A, const T* b, T* x, int64_t max_iter, double
   Scratch sc;
   const size_t vec = ((size_t)n * sizeof(T) + 255) / 256 * 256;
   const size_t pb = ((size_t)upd_blocks * sizeof(double) + 255) / 256 * 256;
-  RVVLA_CUDA(sc.alloc(6 * vec + 2 * pb + sizeof(BiScalars), st));
+  RVVLA_CUDA(sc.alloc_kept(6 * vec + 2 * pb + sizeof(BiScalars), st));
   char* base = sc.as<char>();
   T* r = reinterpret_cast<T*>(base);
   T* rh = reinterpret_cast<T*>(base + vec);

@@ -293,7 +293,7 @@ int vhcc_spmv_impl(const rvvla_vhcc* A, X alpha, const X* x, X beta, X* y, cudaS
   if (rc) return rc;
   if (A->num_rows == 0) return RVVLA_OK;
   Scratch sc;
-  RVVLA_CUDA(sc.alloc((size_t)A->pad_rows * sizeof(CT), st));
+  RVVLA_CUDA(sc.alloc_kept((size_t)A->pad_rows * sizeof(CT), st));
   CT* tmp = sc.as<CT>();
   RVVLA_CUDA(cudaMemsetAsync(tmp, 0, (size_t)A->pad_rows * sizeof(CT), st));
   const int64_t NT = A->num_threads;

@@ -158,7 +158,7 @@ int vnec_spmv_impl(const rvvla_vnec* A, X alpha, const X* x, X beta, X* y, cudaS
       return fail(RVVLA_ERR_UNSUPPORTED, "vnec: a thread's compacted x exceeds 200 KB of shared memory; build with more threads");
     if (A->vnec_t == 0) {
       Scratch sc;
-      RVVLA_CUDA(sc.alloc((size_t)NT * (sizeof(int) + sizeof(CT)) + 256, st));
+      RVVLA_CUDA(sc.alloc_kept((size_t)NT * (sizeof(int) + sizeof(CT)) + 256, st));
       int* crow = sc.as<int>();
       CT* cval = reinterpret_cast<CT*>(sc.as<char>() + ((size_t)NT * sizeof(int) + 255) / 256 * 256);
       auto k_ = vnec_d_kernel<V, X, CT>;
@@ -194,13 +194,13 @@ int vnec_spmv_impl(const rvvla_vnec* A, X alpha, const X* x, X beta, X* y, cudaS
   int32_t* plan;
   if (ipt <= tile) {
     ntiles = NT;
-    RVVLA_CUDA(sc.alloc((size_t)(2 * (NT + 1)) * sizeof(int32_t) + (size_t)NT * (sizeof(int) + sizeof(CT)) + 512, st));
+    RVVLA_CUDA(sc.alloc_kept((size_t)(2 * (NT + 1)) * sizeof(int32_t) + (size_t)NT * (sizeof(int) + sizeof(CT)) + 512, st));
     plan = sc.as<int32_t>();
     vnec_plan_kernel<<<(NT + 255) / 256, 256, 0, st>>>(NT, A->thread_coord_start, A->thread_coord_end, plan);
     RVVLA_LAUNCHED("vnec_plan_kernel");
   } else {
     ntiles = crs_tiles(A->m, A->nz, IPT);
-    RVVLA_CUDA(sc.alloc((size_t)(2 * (ntiles + 1)) * sizeof(int32_t) + (size_t)ntiles * (sizeof(int) + sizeof(CT)) + 512, st));
+    RVVLA_CUDA(sc.alloc_kept((size_t)(2 * (ntiles + 1)) * sizeof(int32_t) + (size_t)ntiles * (sizeof(int) + sizeof(CT)) + 512, st));
     plan = sc.as<int32_t>();
     rc = crs_plan_launch(A->m, A->nz, A->ptr, IPT, plan, st);
     if (rc) return rc;
