@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "crs_merge.cuh"
 #include "rvvla_internal.cuh"
@@ -127,84 +128,114 @@ sell_spmv_kernel(int64_t m, int64_t C, const int* __restrict__ vCl, const int* _
 // coalesced).  A CTA covers 8 consecutive slices; slices wider than
 // kSellWide columns (the long rows that sigma-sorting gathers at the head of
 // a window) are shared by all 8 warps of the CTA, each taking every eighth
-// group of 4 columns, and the 8 partial sums of a row are merged in warp
-// order through shared memory, so a wide slice costs the CTA width/8 steps
-// instead of holding one warp for width steps.
+// group of columns, and the 8 partial sums of a row are merged in warp
+// order through shared memory, so a wide slice costs the CTA width / (8 U)
+// steps instead of holding one warp for width / U steps.
+//
+// Bound by latency, not by the padding's bytes (skipping loads past a row's
+// end did not lower DRAM reads: lines come whole): a slice's last columns one
+// at a time cost a trip to memory each, and conditional loads in the wide
+// slices went out one by one.  Every group of columns now leaves together, the
+// CTA's widths are one load, and registers are sized for five CTAs per SM (with
+// eight the compiler interleaved loads and uses).  Power law 4M: fp32 332 -> 284
+// us, fp64 483 -> 428, mixed fp32 376 -> 318; 2M bf16 232 -> 157; 100K fp64 32 ->
+// 20; stencil 128^3 fp32 92 -> 82; Laplacian 1500^2 fp64 41 -> 38.
 constexpr int kSellWide = 64;
+constexpr int kSellWarps = 8;
+
+// Columns j, j + step, .. (below w) of the lane's row added to acc, U at a
+// time; the columns left over one at a time (ONES; better for short groups of
+// 8-byte values: the 5 columns of a Laplacian took 45 us as two groups, 38), or
+// in one group whose loads past the slice repeat its last column.
+template <int U, bool ONES, class V, class X, class Ac>
+__device__ __forceinline__ void sell_columns(Ac& acc, const uint32_t* __restrict__ col, const V* __restrict__ val,
+                                             int bs, int j, int step, int w, const X* __restrict__ x, uint64_t pf,
+                                             uint64_t pl) {
+  // plain fp32 sums the odd columns apart, which halves a long chain of roundings
+  constexpr bool TWO = std::is_same<Ac, float>::value;
+  Ac odd;
+  acc_zero(odd);
+  for (; j + U <= w; j += step) {
+    uint32_t c[U];
+    V v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      c[u] = ld_stream(col + (int64_t)(j + u) * bs, pf);
+      v[u] = ld_stream(val + (int64_t)(j + u) * bs, pf);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc_add(TWO && (u & 1) ? odd : acc, vmul(v[u], ld_keep(x + c[u], pl)));
+  }
+  if constexpr (ONES) {
+    for (const int end = min(w, j + U); j < end; ++j) {
+      const uint32_t c = ld_stream(col + (int64_t)j * bs, pf);
+      acc_add(acc, vmul(ld_stream(val + (int64_t)j * bs, pf), ld_keep(x + c, pl)));
+    }
+  } else if (j < w) {
+    uint32_t c[U];
+    V v[U];
+    X xv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t k = (int64_t)min(j + u, w - 1) * bs;
+      c[u] = ld_stream(col + k, pf);
+      v[u] = ld_stream(val + k, pf);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) xv[u] = ld_keep(x + c[u], pl);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (j + u < w) acc_add(TWO && (u & 1) ? odd : acc, vmul(v[u], xv[u]));
+  }
+  if (TWO) acc_merge(acc, odd);
+}
 
 template <class V, class X, class Ac, int MODE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * kSellWarps, 5)
 sell_warp_kernel(int64_t cnt_b, const int* __restrict__ vCl, const int* __restrict__ vCs,
                  const int* __restrict__ vBs, const int* __restrict__ vSBs, const uint32_t* __restrict__ vCol,
                  const uint32_t* __restrict__ vPerm, const V* __restrict__ vVal, const X* __restrict__ x,
                  X* __restrict__ y, X alpha, X beta) {
-  __shared__ Ac red[8][32];
+  constexpr int W = kSellWarps;
+  constexpr int U = sizeof(V) >= 8 ? 4 : 8;                   // columns in flight
+  constexpr int UW = std::is_same<Ac, float>::value ? 16 : 8;  // the same in a wide slice
+  __shared__ Ac red[W][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t s0 = (int64_t)blockIdx.x * 8;
+  const int64_t s0 = (int64_t)blockIdx.x * W;
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
-  {
+  const int wq = lane < W && s0 + lane < cnt_b ? vCl[s0 + lane] : 0;  // the CTA's widths
+  auto store = [&](int64_t s, int bs, const Ac& acc) {
+    if (lane >= bs) return;
+    const int64_t out = (MODE == 1) ? (int64_t)vPerm[vSBs[s] + lane] : (int64_t)vSBs[s] + lane;
+    write_row(y, (int)out, alpha, beta, (X)acc_out(acc));
+  };
+  if (s0 + warp < cnt_b) {
     const int64_t s = s0 + warp;
-    if (s < cnt_b) {
-      const int w = vCl[s], bs = vBs[s];
-      if (w <= kSellWide && lane < bs) {
-        const int64_t base = vCs[s] + lane;
-        Ac acc;
-        acc_zero(acc);
-        // columns in flight: 4 for 8-byte values, 8 for narrower ones
-        constexpr int U = sizeof(V) >= 8 ? 4 : 8;
-        int j = 0;
-        for (; j + U <= w; j += U) {
-          uint32_t c[U];
-          V v[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            c[u] = ld_stream(vCol + base + (int64_t)(j + u) * bs, pf);
-            v[u] = ld_stream(vVal + base + (int64_t)(j + u) * bs, pf);
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) acc_add(acc, vmul(v[u], ld_keep(x + c[u], pl)));
-        }
-        for (; j < w; ++j) {
-          const uint32_t c = ld_stream(vCol + base + (int64_t)j * bs, pf);
-          acc_add(acc, vmul(ld_stream(vVal + base + (int64_t)j * bs, pf), ld_keep(x + c, pl)));
-        }
-        const int64_t out = (MODE == 1) ? (int64_t)vPerm[vSBs[s] + lane] : (int64_t)vSBs[s] + lane;
-        write_row(y, (int)out, alpha, beta, (X)acc_out(acc));
-      }
+    const int w = __shfl_sync(0xffffffffu, wq, warp), bs = vBs[s];
+    if (w <= kSellWide) {
+      const int64_t base = vCs[s] + min(lane, bs - 1);  // lanes beyond a short slice repeat its last row
+      Ac acc;
+      acc_zero(acc);
+      sell_columns<U, sizeof(V) >= 8>(acc, vCol + base, vVal + base, bs, 0, U, w, x, pf, pl);
+      store(s, bs, acc);
     }
   }
-  for (int q = 0; q < 8; ++q) {  // wide slices: the whole CTA (uniform branches)
+  // wide slices: the whole CTA (the mask is the same in all warps)
+  for (unsigned wide = __ballot_sync(0xffffffffu, wq > kSellWide); wide; wide &= wide - 1) {
+    const int q = __ffs(wide) - 1;
     const int64_t s = s0 + q;
-    if (s >= cnt_b) break;
-    const int w = vCl[s];
-    if (w <= kSellWide) continue;
-    const int bs = vBs[s];
+    const int w = __shfl_sync(0xffffffffu, wq, q), bs = vBs[s];
+    const int64_t base = vCs[s] + min(lane, bs - 1);
     Ac acc;
     acc_zero(acc);
-    if (lane < bs) {
-      const int64_t base = vCs[s] + lane;
-      for (int j0 = warp * 4; j0 < w; j0 += 32) {
-        uint32_t c[4];
-        V v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const bool in = j0 + u < w;
-          c[u] = in ? ld_stream(vCol + base + (int64_t)(j0 + u) * bs, pf) : 0u;
-          v[u] = in ? ld_stream(vVal + base + (int64_t)(j0 + u) * bs, pf) : V(0.0f);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (j0 + u < w) acc_add(acc, vmul(v[u], ld_keep(x + c[u], pl)));
-      }
-    }
+    sell_columns<UW, false>(acc, vCol + base, vVal + base, bs, warp * UW, W * UW, w, x, pf, pl);
     red[warp][lane] = acc;
     __syncthreads();
-    if (warp == 0 && lane < bs) {
+    if (warp == 0) {
       Ac t = red[0][lane];
 #pragma unroll
-      for (int k = 1; k < 8; ++k) acc_merge(t, red[k][lane]);
-      const int64_t out = (MODE == 1) ? (int64_t)vPerm[vSBs[s] + lane] : (int64_t)vSBs[s] + lane;
-      write_row(y, (int)out, alpha, beta, (X)acc_out(t));
+      for (int k = 1; k < W; ++k) acc_merge(t, red[k][lane]);
+      store(s, bs, t);
     }
     __syncthreads();
   }
@@ -247,12 +278,12 @@ int sell_spmv_impl(const rvvla_sell* A, int stage, X alpha, const X* x, X beta, 
   }
   const V* vv = (const V*)A->vVal;
   if (A->C == 32 && (stage == RVVLA_STAGE_MULT || stage == RVVLA_STAGE_ALL)) {
-    const unsigned wblocks = (unsigned)((A->cnt_b + 7) / 8);
+    const unsigned wblocks = (unsigned)((A->cnt_b + kSellWarps - 1) / kSellWarps);
     if (stage == RVVLA_STAGE_MULT)
-      sell_warp_kernel<V, X, Ac, 0><<<wblocks, 256, 0, st>>>(A->cnt_b, A->vCl, A->vCs, A->vBs, A->vSBs, A->vCol,
+      sell_warp_kernel<V, X, Ac, 0><<<wblocks, 32 * kSellWarps, 0, st>>>(A->cnt_b, A->vCl, A->vCs, A->vBs, A->vSBs, A->vCol,
                                                              A->vPerm, vv, x, y, alpha, beta);
     else
-      sell_warp_kernel<V, X, Ac, 1><<<wblocks, 256, 0, st>>>(A->cnt_b, A->vCl, A->vCs, A->vBs, A->vSBs, A->vCol,
+      sell_warp_kernel<V, X, Ac, 1><<<wblocks, 32 * kSellWarps, 0, st>>>(A->cnt_b, A->vCl, A->vCs, A->vBs, A->vSBs, A->vCol,
                                                              A->vPerm, vv, x, y, alpha, beta);
     RVVLA_LAUNCHED("sell_warp_kernel");
     return RVVLA_OK;
