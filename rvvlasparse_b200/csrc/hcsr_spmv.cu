@@ -7,12 +7,15 @@
 // C are accepted (the only limits are the format's: uint16 local columns,
 // 30-bit row_ptr offsets).
 //
-// GPU mapping.  One CTA of 16 warps per block row; the block row's R partial
-// sums live in shared memory (or, for block rows too tall for shared memory,
-// in a global scratch slice the CTA owns).  Every row belongs to one warp:
-// warp w owns rows [ceil(w*rows/16), ceil((w+1)*rows/16)), so no two warps
-// ever add into the same row and the summation order of every row is fixed —
-// the result is bitwise reproducible run to run (no float atomics).
+// GPU mapping.  A block row belongs to one CTA of 8 warps, or, where there are
+// fewer block rows than the device holds CTAs, to a cluster of up to 8 (its
+// parts, hcsr_split); each CTA's R partial sums live in its shared memory (or,
+// for block rows too tall for it, in a global scratch slice the one CTA owns).
+// In the row-range phase every row belongs to one of the block row's warps: of
+// W warps, warp w owns rows [ceil(w*rows/W), ceil((w+1)*rows/W)); in the COO
+// phase the warps of a CTA add in turn.  The summation order of every row is
+// therefore fixed and the result bitwise reproducible run to run (no float
+// atomics).
 //
 // The block columns are taken in windows of kHWin blocks: the window's
 // non-empty blocks are compacted into a row-range list and a COO list in
@@ -31,27 +34,34 @@
 //     the same way, a row starting wherever the row changes; a CTA that finds
 //     rows out of order there starts its block row over with every COO block
 //     in the COO phase;
-//   * COO phase: the window's other COO nonzeros (in block order) are cut
-//     into rounds of 1024; every warp computes 64 products in stream order
-//     (the block of each nonzero from the compacted list: a warp-wide OR of
-//     the next block starts and a popcount), writes (row, product, owner) to
-//     shared memory — a run of one row inside one block summed first, by a
-//     segmented warp scan — and after a barrier each owner warp picks its own
-//     run sums in stream order and adds them 32 at a time (COO rows belong to
-//     warps in interleaved chunks of 16 rows, so that the few hundred
-//     consecutive rows of a block spread over the warps; the row-range
-//     phase's ranges are not needed here, since barriers separate the
-//     phases); lanes holding the same row add one after another in lane
-//     order (an integer atomicMin over a per-warp slot table elects the
-//     lowest pending lane of each row per round).
-// The next round's loads are issued before the current round is applied.
+//   * COO phase: the window's other COO nonzeros (in block order; a cluster's
+//     CTAs take consecutive shares of them) are cut into rounds of 512; warp w
+//     takes the w-th 64 of a round, 32 at a time (the block of each nonzero
+//     from the compacted list: a warp-wide OR of the next block starts and a
+//     popcount).  A run of one row inside one block is summed first, by a
+//     segmented warp scan; lanes that hold the same row are ranked by a warp
+//     match.  Then the warp waits for its turn, adds its sums into the rows,
+//     rank by rank, and hands the turn on through a named barrier, so that
+//     every row receives its sums in stream order.  Only the adds lie inside
+//     the turn: loads, gathers, products and ranks of the other warps go on
+//     meanwhile.
 // A COO row index at or beyond the block row's rows (malformed input; the
 // builder never writes one) is skipped rather than written out of range.
-// Per row, the sum is: row-range pieces of window 0 in block order, COO
-// products of window 0 in stream order, then window 1, ...; y = alpha*acc +
-// beta*y at the end (y is not read when beta == 0).  Shared memory is sized
-// for two CTAs per SM and the carveout asks for no more, so that the rest of
-// the SM's 256 KB serves as L1 for the gathers of x.
+// Per row and part, the sum is: row-range pieces of window 0 in block order,
+// COO sums of window 0 in stream order, then window 1, ...; the parts are added
+// in order, and y = alpha*sum + beta*y (y is not read when beta == 0).
+//
+// What bounds it: the latency of the chain list -> row/column -> x in both
+// phases, at 32 warps per SM (issue slots 41 % busy, LSU 58 %, DRAM 16 % on the
+// power law of 1M rows, 19.6M nonzeros, R = C = 2000, fp64).  COO products
+// that went through shared memory to the warp that owns their row, which
+// filtered them out of each round, cost 350 instructions per 32 nonzeros and a
+// barrier per round, with 16-warp CTAs: 223 us; in turns 149, and 141 with the
+// carveout at the size the CTAs need (uniformly random columns 447 -> 244, the
+// power law of 2M rows 454 -> 294, stencil 100^3, all CSR blocks, 129 -> 110).
+// A turn of 32 nonzeros takes 162 us for the first, one of 128 149 (64: 149).
+// Shared memory is sized for four CTAs per SM and the carveout asks for no
+// more, so that the rest of the SM's 256 KB serves as L1 for the gathers of x.
 //
 // Mixed forms: lane sums of the CSR phase in compensated fp32 (two-sum), COO
 // products in fp32; the block-row accumulator, where pieces of different
@@ -69,21 +79,19 @@ namespace rvvla {
 namespace {
 
 constexpr uint32_t kHKindMask = 0x3FFFFFFFu;
-constexpr int kHW = 16;                    // warps per CTA = row owners
+constexpr int kHW = 8;                     // warps per CTA
 constexpr int kHT = 32 * kHW;              // threads per CTA
-constexpr int kHMinBlocks = 2;             // resident CTAs per SM the registers are sized for
-constexpr int kHWLog = kHW == 8 ? 3 : 4;
-static_assert(kHW == 8 || kHW == 16, "8 or 16 row owners");
+constexpr int kHMinBlocks = 4;             // resident CTAs per SM the registers are sized for
 constexpr int kHPer = 1;                   // block columns per thread in a window
 constexpr int kHWin = kHPer * kHT;         // block columns per window
-constexpr int kHRound = 1024;              // COO nonzeros per round
-constexpr int kHU = kHRound / (kHW * 32);  // sub-steps of 32 per warp and round
-constexpr int kHStages = 2;                // COO stage buffers (round t fills t % kHStages)
-constexpr int kHSlots = 2048 / kHW;        // per-warp row slots of the COO apply (power of two)
+constexpr int kHProbe = kHWin / 32;        // list entries between the first probes of a search
+static_assert(kHProbe >= 1 && kHProbe <= 32, "two steps of 32 probes reach every list entry");
+constexpr int kHU = 2;                     // sub-steps of 32 COO nonzeros in a warp's turn
+constexpr int kHRound = kHW * kHU * 32;    // COO nonzeros of one turn of every warp
+static_assert(kHW <= 15, "one named barrier per warp beside barrier 0");
 constexpr int kHBig = 1024;                // COO blocks of at least this many nonzeros take the row-range path
 constexpr int kHLane = 8;                  // CSR nonzeros per lane and chunk
 constexpr int kHChunk = 32 * kHLane;
-constexpr int kHWscr = kHChunk * 4 > 1024 ? kHChunk * 4 : 1024;  // per-warp scratch bytes
 
 // a non-empty block of the window: COO stream start (COO list only), nonzero
 // offset, row_ptr offset, block column
@@ -97,21 +105,16 @@ static_assert(sizeof(HBlk) == 16, "HBlk is one 16-byte shared-memory load");
 
 __host__ __device__ constexpr size_t hal16(size_t b) { return (b + 15) / 16 * 16; }
 
-// Dynamic shared memory: [acc] list | prod | row | own | per-warp scratch |
-// per-warp mark groups.
-template <class SA, class P>
+// Dynamic shared memory: [acc] list | per-warp row marks | per-warp mark groups.
+template <class SA>
 struct HLayout {
-  size_t acc, list, prod, row, own, wscr, mgrp, slot, total;
+  size_t acc, list, mark, mgrp, total;
   __host__ __device__ explicit HLayout(int64_t racc) {
     acc = 0;
     list = hal16((size_t)racc * sizeof(SA));
-    prod = list + hal16((size_t)(kHWin + 1) * sizeof(HBlk));
-    row = prod + hal16((size_t)kHStages * kHRound * sizeof(P));
-    own = row + (size_t)kHStages * kHRound * 4;
-    wscr = own + hal16((size_t)kHStages * kHRound);
-    mgrp = wscr + (size_t)kHW * kHWscr;
-    slot = mgrp + (size_t)kHW * 32 * 4;
-    total = slot + (size_t)kHW * kHSlots * 4;
+    mark = list + hal16((size_t)(kHWin + 1) * sizeof(HBlk));
+    mgrp = mark + (size_t)kHW * kHChunk * 4;
+    total = mgrp + (size_t)kHW * 32 * 4;
   }
 };
 
@@ -122,13 +125,13 @@ struct HTypes {
   using PT = decltype(vmul(V(), X()));              // a product
 };
 
-// COO rows belong to warps in chunks of 16 consecutive rows, interleaved
-// (a block of a few hundred consecutive rows spreads over the warps)
-__device__ __forceinline__ uint32_t hcsr_coo_owner(uint32_t r) { return (r >> 4) & (kHW - 1); }
-// the slot of an owned row in its warp's table: distinct for 16 * kHSlots
-// consecutive rows
-__device__ __forceinline__ uint32_t hcsr_coo_slot(uint32_t r) {
-  return (((r >> (4 + kHWLog)) << 4) | (r & 15)) & (kHSlots - 1);
+// The turns of the warps: a warp waits on its own barrier for the warp before
+// it, and hands on by arriving at the next warp's.
+__device__ __forceinline__ void hcsr_turn_wait(int warp) {
+  asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + warp) : "memory");
+}
+__device__ __forceinline__ void hcsr_turn_pass(int warp) {
+  asm volatile("barrier.cta.arrive %0, 64;" ::"r"(1 + (warp + 1) % kHW) : "memory");
 }
 
 // Exclusive CTA-wide scan of three counters; t* are the CTA totals.
@@ -173,7 +176,6 @@ __device__ __forceinline__ void hcsr_scan3(int a, int b, int c, int& pa, int& pb
   __syncthreads();
 }
 
-// eight uint16 columns with one 16-byte load
 // kHLane uint16 columns with 16-byte loads
 __device__ __forceinline__ void hcsr_cols(const uint16_t* p, uint32_t (&c)[kHLane], uint64_t pol) {
 #pragma unroll
@@ -499,6 +501,27 @@ __device__ __forceinline__ bool hcsr_coo_rows(const uint32_t* __restrict__ rp, i
   return bad;
 }
 
+// Barrier of the CTAs that share a block row; shared memory written before it
+// is visible to them after it.
+__device__ __forceinline__ void hcsr_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The shared-memory address of p in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t hcsr_peer(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void hcsr_peer_ld(uint32_t a, int& v) {
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void hcsr_peer_ld(uint32_t a, float& v) {
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void hcsr_peer_ld(uint32_t a, double& v) {
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+}
+
 // Raw loads of one COO sub-step (32 consecutive COO nonzeros of the window).
 template <class V>
 struct HCooRaw {
@@ -509,40 +532,37 @@ struct HCooRaw {
   bool ok;
 };
 
-template <class V, class X, class SA, bool MIX, bool VEC, bool GACC>
+template <class V, class X, class SA, bool MIX, bool VEC, bool GACC, bool SPLIT>
 __global__ void __launch_bounds__(kHT, kHMinBlocks)
 hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const int* __restrict__ block_ptr,
                  const uint32_t* __restrict__ row_offset, const uint32_t* __restrict__ row_ptr,
                  const uint16_t* __restrict__ col_idx, const V* __restrict__ values, const X* __restrict__ x,
-                 X* __restrict__ y, X alpha, X beta, SA* __restrict__ gacc) {
+                 X* __restrict__ y, X alpha, X beta, SA* __restrict__ gacc, int parts) {
   using Ty = HTypes<V, X, SA, MIX>;
   using P = typename Ty::P;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_w[3 * kHW];
-  const HLayout<SA, P> L(GACC ? 0 : min(R, m));  // as the launch sizes it
+  const HLayout<SA> L(GACC ? 0 : min(R, m));  // as the launch sizes it
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t br = blockIdx.x;
+  const int split = SPLIT ? parts : 1;  // CTAs (one cluster) that share a block row
+  const int64_t br = blockIdx.x / (unsigned)split;
+  const int part = (int)(blockIdx.x % (unsigned)split);
   const int64_t r0 = br * R;
   const int rows = (int)min(R, m - r0);
   SA* acc = GACC ? gacc + r0 : reinterpret_cast<SA*>(smem + L.acc);
   HBlk* list = reinterpret_cast<HBlk*>(smem + L.list);
-  P* s_prod0 = reinterpret_cast<P*>(smem + L.prod);
-  uint32_t* s_row0 = reinterpret_cast<uint32_t*>(smem + L.row);
-  uint8_t* s_own0 = smem + L.own;
-  int* table = reinterpret_cast<int*>(smem + L.wscr + (size_t)warp * kHWscr);          // CSR phase
-  uint16_t* olist = reinterpret_cast<uint16_t*>(smem + L.wscr + (size_t)warp * kHWscr);  // COO phase
+  int* table = reinterpret_cast<int*>(smem + L.mark) + warp * kHChunk;
   uint32_t* mgrp = reinterpret_cast<uint32_t*>(smem + L.mgrp) + warp * 32;
   __shared__ int s_bad;  // a large COO block whose rows do not ascend was met
   bool big_ok = true;
-  int* slot = reinterpret_cast<int*>(smem + L.slot) + warp * kHSlots;
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
 
   for (int li = tid; li < rows; li += kHT) acc[li] = SA(0);
-  for (int q = lane; q < kHSlots; q += 32) slot[q] = INT_MAX;
   if (tid == 0) s_bad = 0;
   // this warp's rows
-  const int ra = (int)(((int64_t)warp * rows + kHW - 1) / kHW);
-  const int rb = (int)(((int64_t)(warp + 1) * rows + kHW - 1) / kHW);
+  const int owner = part * kHW + warp, owners = split * kHW;
+  const int ra = (int)(((int64_t)owner * rows + owners - 1) / owners);
+  const int rb = (int)(((int64_t)(owner + 1) * rows + owners - 1) / owners);
   const int64_t blk0 = br * b_n;
   __syncthreads();
 
@@ -616,8 +636,8 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
                                           mgrp, lane, pf, pl);
       } else {
         const int cnt = h.cs;
-        const int klo = warp == 0 ? 0 : hcsr_lower_bound(rp, cnt, (uint32_t)ra, lane);
-        const int khi = warp == kHW - 1 ? cnt : hcsr_lower_bound(rp, cnt, (uint32_t)rb, lane);
+        const int klo = owner == 0 ? 0 : hcsr_lower_bound(rp, cnt, (uint32_t)ra, lane);
+        const int khi = owner == owners - 1 ? cnt : hcsr_lower_bound(rp, cnt, (uint32_t)rb, lane);
         if (klo > khi) {
           if (lane == 0) s_bad = 1;
           continue;
@@ -630,24 +650,22 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
     }
 
     // ---- COO phase: rounds of kHRound nonzeros of the window's COO stream
-    if (t_ent > 0) {
-      const int ncoo = t_coo, ntot = t_ent;
-      const int nrounds = (ntot + kHRound - 1) / kHRound;
+    // (this CTA's share: nonzeros [qlo, ntot) of it)
+    const int share = ((t_ent + split - 1) / split + 31) & ~31;
+    const int qlo = min(part * share, t_ent);
+    if (qlo < t_ent && share > 0) {
+      const int ncoo = t_coo, ntot = min(qlo + share, t_ent);
+      const int nrounds = (ntot - qlo + kHRound - 1) / kHRound;
       HCooRaw<V> raw[kHU];
       auto coo_load = [&](int t) {
-        const int q00 = t * kHRound + warp * (kHU * 32);
-        int ia = 0;
-        if (lane == 0) {
-          const int qs = min(q00, ntot - 1);
-          int lo = 0, hi = ncoo;
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (list[mid].cs <= qs) lo = mid;
-            else hi = mid;
-          }
-          ia = lo;
-        }
-        ia = __shfl_sync(0xffffffffu, ia, 0);
+        const int q00 = qlo + t * kHRound + warp * (kHU * 32);
+        // the block of the warp's first nonzero: the last that starts at or
+        // before it, by two steps of 32 probes (list[0].cs is 0)
+        const int qs = min(q00, ntot - 1);
+        int ia = lane * kHProbe < ncoo && list[lane * kHProbe].cs <= qs;
+        ia = kHProbe * (__popc(__ballot_sync(0xffffffffu, ia)) - 1);
+        const bool le = lane < kHProbe && ia + lane < ncoo && list[ia + lane].cs <= qs;
+        ia += __popc(__ballot_sync(0xffffffffu, le)) - 1;
 #pragma unroll
         for (int u = 0; u < kHU; ++u) {
           const int q0 = q00 + 32 * u;
@@ -675,19 +693,16 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
         }
       };
       coo_load(0);
+      __syncthreads();  // the row-range phase of every warp is over
       for (int t = 0; t < nrounds; ++t) {
-        // this round's stage buffer: with two, round t + 1 is produced while
-        // slower warps still apply round t, and one barrier per round does
-        P* const s_prod = s_prod0 + (t % kHStages) * kHRound;
-        uint32_t* const s_row = s_row0 + (t % kHStages) * kHRound;
-        uint8_t* const s_own = s_own0 + (t % kHStages) * kHRound;
-        // products of this round into shared memory, in stream order
         X xv[kHU];
 #pragma unroll
         for (int u = 0; u < kHU; ++u) xv[u] = raw[u].ok ? ld_keep(x + raw[u].xoff + raw[u].col, pl) : X(0);
+        uint32_t row[kHU];
+        P pr[kHU];
+        int rank[kHU], last[kHU];
 #pragma unroll
         for (int u = 0; u < kHU; ++u) {
-          const int i = warp * (kHU * 32) + 32 * u + lane;
           const HCooRaw<V>& r = raw[u];
           P pv = P(0);
           if (r.ok) {
@@ -695,99 +710,75 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
             else pv = (P)(r.v * xv[u]);
           }
           // runs of one row inside one block (consecutive lanes) are summed
-          // here; only the run's last lane is handed on
+          // here, into the run's last lane
           // (cont: this lane continues the previous lane's run; most
           // sub-steps have none, and skip the scan)
           const uint32_t prow = __shfl_up_sync(0xffffffffu, r.row, 1);
           const int64_t pxo = __shfl_up_sync(0xffffffffu, r.xoff, 1);
           const bool cont = lane > 0 && r.ok && prow == r.row && pxo == r.xoff;
-          P run = pv;
           bool tail = r.ok;
           if (__any_sync(0xffffffffu, cont)) {
-            run = warp_seg_scan(pv, !cont, lane);
+            pv = warp_seg_scan(pv, !cont, lane);
             const bool ncont = __shfl_down_sync(0xffffffffu, cont, 1);
             tail = r.ok && (lane == 31 || !ncont);
           }
-          s_prod[i] = run;
-          s_row[i] = r.row;
-          s_own[i] = (uint8_t)(tail ? hcsr_coo_owner(r.row) : 0xFFu);
+          // lanes that hold the same row add one after another, in lane order
+          row[u] = r.row;
+          pr[u] = pv;
+          const unsigned peers = __match_any_sync(0xffffffffu, tail ? row[u] : 0xFFFFFFFFu);
+          rank[u] = tail ? __popc(peers & ((1u << lane) - 1u)) : -1;
+          last[u] = __reduce_max_sync(0xffffffffu, rank[u]);
         }
-        __syncthreads();
         if (t + 1 < nrounds) coo_load(t + 1);
-        // this warp's nonzeros of the round, in stream order
-        const uint32_t me = (uint32_t)warp * 0x01010101u;
-#pragma unroll 1
-        for (int it = 0; it < kHRound / 512; ++it) {
-          const uint4 w4 = reinterpret_cast<const uint4*>(s_own)[it * 32 + lane];
-          const uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
-          uint32_t m16 = 0;
+        // the warps take turns, so every row receives its sums in stream order
+        if (t > 0 || warp > 0) hcsr_turn_wait(warp);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t eq = __vcmpeq4(ws[q], me);
-            m16 |= (((eq >> 7) & 1u) | ((eq >> 14) & 2u) | ((eq >> 21) & 4u) | ((eq >> 28) & 8u)) << (4 * q);
-          }
-          const int cnt = __popc(m16);
-          int inc = cnt;
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const int o = __shfl_up_sync(0xffffffffu, inc, d);
-            if (lane >= d) inc += o;
-          }
-          const int total = __shfl_sync(0xffffffffu, inc, 31);
-          int pos = inc - cnt;
-          while (m16) {
-            const int b = __ffs(m16) - 1;
-            olist[pos++] = (uint16_t)(it * 512 + 16 * lane + b);
-            m16 &= m16 - 1u;
-          }
-          __syncwarp();
-          // groups of 32 of this warp's nonzeros; inside a group, rounds in
-          // which the lowest pending lane of every row slot adds its value
-          // (an integer atomicMin elects it), so each row receives its
-          // values in lane order = stream order, whatever the scheduling
-          for (int g = 0; g < total; g += 32) {
-            const int tt = g + lane;
-            bool pend = tt < total;
-            uint32_t r = 0;
-            SA pv = SA(0);
-            if (pend) {
-              const int i = olist[tt];
-              r = s_row[i];
-              pv = (SA)s_prod[i];
-            }
-            int* sl = slot + hcsr_coo_slot(r);
-            while (__ballot_sync(0xffffffffu, pend)) {
-              if (pend) atomicMin(sl, lane);
-              __syncwarp();
-              const bool win = pend && *sl == lane;
-              __syncwarp();
-              if (win) {
-                acc[r] += pv;
-                *sl = INT_MAX;
-                pend = false;
-              }
-              __syncwarp();
-            }
+        for (int u = 0; u < kHU; ++u) {
+          for (int k = 0; k <= last[u]; ++k) {
+            if (rank[u] == k) acc[row[u]] += pr[u];
+            __syncwarp();
           }
         }
-        if (kHStages == 1) __syncthreads();
+        if (t + 1 < nrounds || warp + 1 < kHW) hcsr_turn_pass(warp);
       }
     }
     __syncthreads();
   }
-  if (!big_ok || !s_bad) break;
+  int bad = s_bad;
+  if constexpr (SPLIT) {
+    hcsr_cluster_sync();  // every CTA's sums of the block row are complete
+    for (int k = 0; k < split; ++k) {
+      int b;
+      hcsr_peer_ld(hcsr_peer(&s_bad, k), b);
+      bad |= b;
+    }
+  }
+  if (!big_ok || !bad) break;
   // rows of a large COO block out of order: start over, all COO blocks
-  // through the COO stream
+  // through the COO stream (the CTAs of a cluster together)
   big_ok = false;
   __syncthreads();
   for (int li = tid; li < rows; li += kHT) acc[li] = SA(0);
   __syncthreads();
   }
-  for (int li = tid; li < rows; li += kHT) {
-    const X o = (X)acc[li];
+  // the CTAs' sums of a row are added in the order of the parts
+  const int fa = (int)((int64_t)part * rows / split), fb = (int)((int64_t)(part + 1) * rows / split);
+  for (int li = fa + tid; li < fb; li += kHT) {
+    SA sum = SA(0);
+    if constexpr (!SPLIT) {
+      sum = acc[li];
+    } else {
+      for (int k = 0; k < split; ++k) {
+        SA v;
+        hcsr_peer_ld(hcsr_peer(acc + li, k), v);
+        sum += v;
+      }
+    }
+    const X o = (X)sum;
     X* yp = y + r0 + li;
     *yp = (beta == X(0)) ? alpha * o : alpha * o + beta * *yp;
   }
+  if constexpr (SPLIT) hcsr_cluster_sync();  // no CTA leaves while its sums are read
 }
 
 int hcsr_validate(const rvvla_hcsr* A, const void* x, const void* y) {
@@ -804,19 +795,50 @@ int hcsr_validate(const rvvla_hcsr* A, const void* x, const void* y) {
   return RVVLA_OK;
 }
 
+constexpr int64_t kHSplitMax = 8;                           // portable cluster size
+constexpr int64_t kHSplitCtas = (int64_t)kHMinBlocks * 148;  // CTAs the device holds
+constexpr int64_t kHSplitNz = 2048;                         // nonzeros a part keeps at least
+
+// CTAs per block row: as many as keep all CTAs resident at once (cluster
+// sizes need not be powers of two).  Each part walks the block list and row
+// pointers again, so more CTAs than that lose (1M rows in 501 block rows,
+// measured with 16-warp CTAs, two per SM: 1, 2, 4 parts 191, 215, 279 us) and
+// fewer leave SMs idle (power law, fp64, 100K rows in 50 block rows 67 -> 35
+// us, 300K rows 93 -> 62, 30K rows 60 -> 27; fp32 with R = 4000, 1M rows in 251
+// block rows 166 -> 117).
+int hcsr_split(const rvvla_hcsr* A) {
+  const int64_t s = std::min(kHSplitCtas / A->b_m, A->nz / (A->b_m * kHSplitNz));
+  return (int)std::max<int64_t>(1, std::min(s, kHSplitMax));
+}
+
 // Largest dynamic shared memory one CTA may take (227 KB on sm_100a).
 constexpr size_t kHSmemMax = 227 * 1024;
 
-template <class V, class X, class SA, bool MIX, bool VEC, bool GACC>
-int hcsr_launch(const rvvla_hcsr* A, X alpha, const X* x, X beta, X* y, SA* gacc, size_t smem, cudaStream_t st) {
-  auto kern = hcsr_spmv_kernel<V, X, SA, MIX, VEC, GACC>;
+template <class V, class X, class SA, bool MIX, bool VEC, bool GACC, bool SPLIT>
+int hcsr_launch(const rvvla_hcsr* A, int split, X alpha, const X* x, X beta, X* y, SA* gacc, size_t smem, cudaStream_t st) {
+  auto kern = hcsr_spmv_kernel<V, X, SA, MIX, VEC, GACC, SPLIT>;
   RVVLA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // shared memory for kHMinBlocks CTAs, the rest of the SM's 256 KB as L1
-  // (the gathers of x hit there)
-  const int carve = (int)std::min<size_t>(100, (kHMinBlocks * (smem + 1024) * 100 + kHSmemMax - 1) / kHSmemMax);
+  // shared memory for kHMinBlocks CTAs (1 KB of each is the system's), the
+  // rest of the SM's 256 KB as L1: the gathers of x hit there.  The SM takes
+  // one of a few sizes, and a wish above one of them gets the next.
+  const size_t need = kHMinBlocks * (smem + 2048);
+  int carve = 100;
+  for (const int kb : {196, 164, 132, 100, 64})
+    if (need <= (size_t)kb * 1024) carve = kb * 100 / 228;
   RVVLA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carve));
-  kern<<<(unsigned)A->b_m, kHT, smem, st>>>(A->R, A->C, A->m, A->nz, A->b_n, A->block_ptr, A->row_offset,
-                                            A->row_ptr, A->col_idx, (const V*)A->values, x, y, alpha, beta, gacc);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(A->b_m * split));
+  cfg.blockDim = dim3(kHT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {(unsigned)split, 1, 1};
+  cfg.attrs = &at;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  RVVLA_CUDA(cudaLaunchKernelEx(&cfg, kern, A->R, A->C, A->m, A->nz, A->b_n, (const int*)A->block_ptr,
+                                (const uint32_t*)A->row_offset, (const uint32_t*)A->row_ptr,
+                                (const uint16_t*)A->col_idx, (const V*)A->values, x, y, alpha, beta, gacc, split));
   RVVLA_LAUNCHED("hcsr_spmv_kernel");
   return RVVLA_OK;
 }
@@ -830,18 +852,22 @@ int hcsr_spmv_impl(const rvvla_hcsr* A, X alpha, const X* x, X beta, X* y, cudaS
   if (A->b_m > INT32_MAX) return fail(RVVLA_ERR_TOO_LARGE, "hcsr: more than 2^31 - 1 block rows");
   const bool vec = ((uintptr_t)A->values % 16 == 0) && ((uintptr_t)A->col_idx % 16 == 0);
   const int64_t racc = std::min<int64_t>(A->R, A->m);
-  const size_t smem_s = HLayout<SA, P>(racc).total;
+  const size_t smem_s = HLayout<SA>(racc).total;
   if (smem_s <= kHSmemMax) {
-    return vec ? hcsr_launch<V, X, SA, MIX, true, false>(A, alpha, x, beta, y, nullptr, smem_s, st)
-               : hcsr_launch<V, X, SA, MIX, false, false>(A, alpha, x, beta, y, nullptr, smem_s, st);
+    const int split = hcsr_split(A);
+    if (split > 1)
+      return vec ? hcsr_launch<V, X, SA, MIX, true, false, true>(A, split, alpha, x, beta, y, nullptr, smem_s, st)
+                 : hcsr_launch<V, X, SA, MIX, false, false, true>(A, split, alpha, x, beta, y, nullptr, smem_s, st);
+    return vec ? hcsr_launch<V, X, SA, MIX, true, false, false>(A, 1, alpha, x, beta, y, nullptr, smem_s, st)
+               : hcsr_launch<V, X, SA, MIX, false, false, false>(A, 1, alpha, x, beta, y, nullptr, smem_s, st);
   }
   // block rows too tall for shared memory: the accumulator is a global
   // scratch array (each CTA owns its slice)
   Scratch sc;
   RVVLA_CUDA(sc.alloc_kept((size_t)A->m * sizeof(SA), st));
-  const size_t smem_g = HLayout<SA, P>(0).total;
-  return vec ? hcsr_launch<V, X, SA, MIX, true, true>(A, alpha, x, beta, y, sc.as<SA>(), smem_g, st)
-             : hcsr_launch<V, X, SA, MIX, false, true>(A, alpha, x, beta, y, sc.as<SA>(), smem_g, st);
+  const size_t smem_g = HLayout<SA>(0).total;
+  return vec ? hcsr_launch<V, X, SA, MIX, true, true, false>(A, 1, alpha, x, beta, y, sc.as<SA>(), smem_g, st)
+             : hcsr_launch<V, X, SA, MIX, false, true, false>(A, 1, alpha, x, beta, y, sc.as<SA>(), smem_g, st);
 }
 
 }  // namespace
