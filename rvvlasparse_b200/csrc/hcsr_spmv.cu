@@ -10,7 +10,7 @@
 // GPU mapping.  A block row belongs to one CTA of 8 warps, or, where there are
 // fewer block rows than the device holds CTAs, to a cluster of up to 8 (its
 // parts, hcsr_split); each CTA's R partial sums live in its shared memory (or,
-// for block rows too tall for it, in a global scratch slice the one CTA owns).
+// for block rows too tall for it, in a global scratch slice of its own).
 // In the row-range phase every row belongs to one of the block row's warps: of
 // W warps, warp w owns rows [ceil(w*rows/W), ceil((w+1)*rows/W)); in the COO
 // phase the warps of a CTA add in turn.  The summation order of every row is
@@ -549,7 +549,7 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
   const int part = (int)(blockIdx.x % (unsigned)split);
   const int64_t r0 = br * R;
   const int rows = (int)min(R, m - r0);
-  SA* acc = GACC ? gacc + r0 : reinterpret_cast<SA*>(smem + L.acc);
+  SA* acc = GACC ? gacc + part * m + r0 : reinterpret_cast<SA*>(smem + L.acc);
   HBlk* list = reinterpret_cast<HBlk*>(smem + L.list);
   int* table = reinterpret_cast<int*>(smem + L.mark) + warp * kHChunk;
   uint32_t* mgrp = reinterpret_cast<uint32_t*>(smem + L.mgrp) + warp * 32;
@@ -770,7 +770,8 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
     } else {
       for (int k = 0; k < split; ++k) {
         SA v;
-        hcsr_peer_ld(hcsr_peer(acc + li, k), v);
+        if constexpr (GACC) v = __ldcg(gacc + k * m + r0 + li);
+        else hcsr_peer_ld(hcsr_peer(acc + li, k), v);
         sum += v;
       }
     }
@@ -795,24 +796,28 @@ int hcsr_validate(const rvvla_hcsr* A, const void* x, const void* y) {
   return RVVLA_OK;
 }
 
+// Largest dynamic shared memory one CTA may take: 227 KB on sm_100a, less the
+// static arrays.
+constexpr size_t kHSmemMax = 226 * 1024;
+
 constexpr int64_t kHSplitMax = 8;                           // portable cluster size
-constexpr int64_t kHSplitCtas = (int64_t)kHMinBlocks * 148;  // CTAs the device holds
 constexpr int64_t kHSplitNz = 2048;                         // nonzeros a part keeps at least
 
 // CTAs per block row: as many as keep all CTAs resident at once (cluster
-// sizes need not be powers of two).  Each part walks the block list and row
-// pointers again, so more CTAs than that lose (1M rows in 501 block rows,
+// sizes need not be powers of two; an eighth of the slots is left free, since a
+// cluster lies within a GPC: 113 block rows take 53 us in clusters of 5, 565
+// of 592 slots, and 45 in clusters of 4).  Each part walks the block list and
+// row pointers again, so more CTAs than that lose (1M rows in 501 block rows,
 // measured with 16-warp CTAs, two per SM: 1, 2, 4 parts 191, 215, 279 us) and
 // fewer leave SMs idle (power law, fp64, 100K rows in 50 block rows 67 -> 35
 // us, 300K rows 93 -> 62, 30K rows 60 -> 27; fp32 with R = 4000, 1M rows in 251
-// block rows 166 -> 117).
-int hcsr_split(const rvvla_hcsr* A) {
-  const int64_t s = std::min(kHSplitCtas / A->b_m, A->nz / (A->b_m * kHSplitNz));
+// block rows 166 -> 117; accumulators in scratch, 1M rows, R = 60000, fp64
+// 2317 -> 477).
+int hcsr_split(const rvvla_hcsr* A, size_t smem) {
+  const int64_t per_sm = std::min<int64_t>(kHMinBlocks, (kHSmemMax + 2048) / (smem + 2048));
+  const int64_t s = std::min(sm_count() * per_sm * 7 / 8 / A->b_m, A->nz / (A->b_m * kHSplitNz));
   return (int)std::max<int64_t>(1, std::min(s, kHSplitMax));
 }
-
-// Largest dynamic shared memory one CTA may take (227 KB on sm_100a).
-constexpr size_t kHSmemMax = 227 * 1024;
 
 template <class V, class X, class SA, bool MIX, bool VEC, bool GACC, bool SPLIT>
 int hcsr_launch(const rvvla_hcsr* A, int split, X alpha, const X* x, X beta, X* y, SA* gacc, size_t smem, cudaStream_t st) {
@@ -835,7 +840,7 @@ int hcsr_launch(const rvvla_hcsr* A, int split, X alpha, const X* x, X beta, X* 
   at.id = cudaLaunchAttributeClusterDimension;
   at.val.clusterDim = {(unsigned)split, 1, 1};
   cfg.attrs = &at;
-  cfg.numAttrs = split > 1 ? 1 : 0;
+  cfg.numAttrs = SPLIT ? 1 : 0;
   RVVLA_CUDA(cudaLaunchKernelEx(&cfg, kern, A->R, A->C, A->m, A->nz, A->b_n, (const int*)A->block_ptr,
                                 (const uint32_t*)A->row_offset, (const uint32_t*)A->row_ptr,
                                 (const uint16_t*)A->col_idx, (const V*)A->values, x, y, alpha, beta, gacc, split));
@@ -854,20 +859,21 @@ int hcsr_spmv_impl(const rvvla_hcsr* A, X alpha, const X* x, X beta, X* y, cudaS
   const int64_t racc = std::min<int64_t>(A->R, A->m);
   const size_t smem_s = HLayout<SA>(racc).total;
   if (smem_s <= kHSmemMax) {
-    const int split = hcsr_split(A);
+    const int split = hcsr_split(A, smem_s);
     if (split > 1)
       return vec ? hcsr_launch<V, X, SA, MIX, true, false, true>(A, split, alpha, x, beta, y, nullptr, smem_s, st)
                  : hcsr_launch<V, X, SA, MIX, false, false, true>(A, split, alpha, x, beta, y, nullptr, smem_s, st);
     return vec ? hcsr_launch<V, X, SA, MIX, true, false, false>(A, 1, alpha, x, beta, y, nullptr, smem_s, st)
                : hcsr_launch<V, X, SA, MIX, false, false, false>(A, 1, alpha, x, beta, y, nullptr, smem_s, st);
   }
-  // block rows too tall for shared memory: the accumulator is a global
+  // block rows too tall for shared memory: the accumulators are a global
   // scratch array (each CTA owns its slice)
-  Scratch sc;
-  RVVLA_CUDA(sc.alloc_kept((size_t)A->m * sizeof(SA), st));
   const size_t smem_g = HLayout<SA>(0).total;
-  return vec ? hcsr_launch<V, X, SA, MIX, true, true, false>(A, 1, alpha, x, beta, y, sc.as<SA>(), smem_g, st)
-             : hcsr_launch<V, X, SA, MIX, false, true, false>(A, 1, alpha, x, beta, y, sc.as<SA>(), smem_g, st);
+  const int split = hcsr_split(A, smem_g);
+  Scratch sc;
+  RVVLA_CUDA(sc.alloc_kept((size_t)split * A->m * sizeof(SA), st));
+  return vec ? hcsr_launch<V, X, SA, MIX, true, true, true>(A, split, alpha, x, beta, y, sc.as<SA>(), smem_g, st)
+             : hcsr_launch<V, X, SA, MIX, false, true, true>(A, split, alpha, x, beta, y, sc.as<SA>(), smem_g, st);
 }
 
 }  // namespace

@@ -35,7 +35,7 @@ def _product(m, n, ln, dt, mixed, **prm):
 
 @pytest.mark.parametrize("dt,mixed", [(np.float64, False), (np.float32, False), (np.float32, True)])
 @pytest.mark.parametrize("p", [0.01, 2.0, 1e9])  # all CSR blocks, both kinds, all COO
-@pytest.mark.parametrize("brows", [1, 74, 85, 119, 148, 198, 296, 297])  # 8 (by nonzeros 1..), 8, 6, 4, 4, 2, 2, 1 parts
+@pytest.mark.parametrize("brows", [1, 74, 85, 119, 148, 198, 296, 297])  # 8, 7, 6, 4, 3, 2, 1, 1 parts
 def test_parts_of_a_block_row(brows, p, dt, mixed):
     m, n = brows * 97 - 5, 5003
     rng = np.random.default_rng(brows)
@@ -57,3 +57,11 @@ def test_rows_that_repeat_across_lanes(rows):
     """Narrow blocks (one or two nonzeros of each row): every lane of a
     sub-step holds one of a few rows."""
     _product(rows, 4000, np.full(rows, 3000), np.float64, False, R=8, C=2, p=1e9)
+
+
+@pytest.mark.parametrize("brows", [1, 2, 3])
+@pytest.mark.parametrize("dt,mixed", [(np.float64, False), (np.float32, True)])
+def test_parts_of_a_tall_block_row(brows, dt, mixed):
+    """Accumulators too tall for shared memory: one scratch slice per part."""
+    m = brows * 60000 - 7
+    _product(m, 3001, np.random.default_rng(m).integers(0, 6, m), dt, mixed, R=60000, C=700, p=2.0)
