@@ -52,7 +52,7 @@
 // in order, and y = alpha*sum + beta*y (y is not read when beta == 0).
 //
 // What bounds it: the latency of the chain list -> row/column -> x in both
-// phases, at 32 warps per SM (issue slots 41 % busy, LSU 58 %, DRAM 16 % on the
+// phases, at 32 warps per SM (issue slots 43 % busy, LSU 56 %, DRAM 17 % on the
 // power law of 1M rows, 19.6M nonzeros, R = C = 2000, fp64).  COO products
 // that went through shared memory to the warp that owns their row, which
 // filtered them out of each round, cost 350 instructions per 32 nonzeros and a
