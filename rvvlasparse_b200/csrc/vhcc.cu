@@ -148,8 +148,11 @@ __global__ void vhcc_pack_kernel(int64_t total, int64_t nnz, const int* __restri
 }
 
 // ---------------------------------------------------------------- SpMV
-template <class V, class X, class Ac, class CT>
-__global__ void __launch_bounds__(256)
+// Warps per SM: what the registers allow, 32 in fp64 (DENSE: 40, with fewer
+// registers), 40 in fp32.
+constexpr int kVhccThreads = 128;
+template <class V, class X, class Ac, class CT, bool DENSE>
+__global__ void __launch_bounds__(kVhccThreads, DENSE ? 40 * 32 / kVhccThreads : 1)
 vhcc_spmv_kernel(int64_t NT, int n_eor, int n_rows, const int* __restrict__ thr, const uint32_t* __restrict__ veceor,
                  const uint32_t* __restrict__ smask, const uint32_t* __restrict__ row_arr,
                  const uint32_t* __restrict__ col, const V* __restrict__ vals, const X* __restrict__ x,
@@ -297,7 +300,16 @@ int vhcc_spmv_impl(const rvvla_vhcc* A, X alpha, const X* x, X beta, X* y, cudaS
   CT* tmp = sc.as<CT>();
   RVVLA_CUDA(cudaMemsetAsync(tmp, 0, (size_t)A->pad_rows * sizeof(CT), st));
   const int64_t NT = A->num_threads;
-  vhcc_spmv_kernel<V, X, Ac, CT><<<(unsigned)((NT * 32 + 255) / 256), 256, 0, st>>>(
+  // The VHCC threads' warps do equal work, so those that a first wave leaves
+  // over take a second one: in fp64, 40 warps per SM where they all fit then
+  // (600K random rows, 5566 warps: 105 us with 32 per SM, 96 with 40; power law
+  // of 642K rows 87 and 78), else 32 (power law of 4M rows: 334 and 380).  CTAs
+  // of four warps against eight: fp32 642K rows 55 -> 52 us, fp64 500K 58 -> 56,
+  // 4M 334 -> 336.
+  const bool dense = sizeof(V) == 8 && NT > 32 * (int64_t)sm_count() && NT <= 40 * (int64_t)sm_count();
+  const unsigned blocks = (unsigned)((NT * 32 + kVhccThreads - 1) / kVhccThreads);
+  auto kern = dense ? vhcc_spmv_kernel<V, X, Ac, CT, sizeof(V) == 8> : vhcc_spmv_kernel<V, X, Ac, CT, false>;
+  kern<<<blocks, kVhccThreads, 0, st>>>(
       NT, (int)A->n_eor, (int)A->n_rowarr, A->thr_info, A->veceor_ptr, (const uint32_t*)A->scan_mask, A->row_arr, A->col_arr, (const V*)A->vals_arr, x,
       tmp);
   RVVLA_LAUNCHED("vhcc_spmv_kernel");
