@@ -20,6 +20,7 @@
 #include <string>
 
 #include "rvvla_internal.cuh"
+#include "sddmm_chunks.h"
 
 namespace rvvla {
 namespace {
@@ -68,9 +69,8 @@ __global__ void tr_gather_kernel(int64_t nz, const int* __restrict__ perm, const
 }
 
 constexpr int kSdThreads = 256;
-constexpr int kSdRows = 256;    // rows per CTA
-constexpr int kSdChunk = 4096;  // nonzeros per pass over the row-start bitmap
-constexpr int kSdU = 8;         // nonzeros per thread in flight
+constexpr int kSdRows = 256;  // rows per CTA
+constexpr int kSdU = 8;       // nonzeros per thread in flight
 
 // dv[k] = g[row(k)] * x[Col[k]]: a CTA per 256 consecutive rows.  The g of its
 // non-empty rows are compacted into shared memory; a bitmap marks the
@@ -112,12 +112,12 @@ sddmm_kernel(int64_t m, const int* __restrict__ Rst, const int* __restrict__ Col
     s_g[at] = g[r0 + t];
   }
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
-  for (int c0 = kb / 32 * 32; c0 < ke; c0 += kSdChunk) {
+  for (SddmmChunk ch = sddmm_first(kb, ke); ch.c0 < ke; ch.c0 += kSdChunk) {
     if (t < W) s_bits[t] = 0u;
     __syncthreads();
     int earlier = 0;  // non-empty rows that start before the chunk
     if (t < rows) {
-      const int k = s_start[t] - c0;
+      const int k = s_start[t] - ch.c0;
       earlier = k < 0;
       if (k >= 0 && k < kSdChunk) atomicOr(&s_bits[k >> 5], 1u << (k & 31));
     }
@@ -140,15 +140,12 @@ sddmm_kernel(int64_t m, const int* __restrict__ Rst, const int* __restrict__ Col
       s_before[t] = base;
     }
     __syncthreads();
-    const int end = min(ke - c0, kSdChunk);
+    const int end = ch.end();
     for (int k0 = t; k0 < end; k0 += kSdU * kSdThreads) {
       int c[kSdU];
       T gv[kSdU], xv[kSdU];
 #pragma unroll
-      for (int u = 0; u < kSdU; ++u) {  // loads past the chunk's range repeat its last nonzero
-        const int k = min(k0 + u * kSdThreads, end - 1);
-        c[u] = ld_stream(Col + max(c0 + k, kb), pf);
-      }
+      for (int u = 0; u < kSdU; ++u) c[u] = ld_stream(Col + ch.load(k0 + u * kSdThreads), pf);
 #pragma unroll
       for (int u = 0; u < kSdU; ++u) {
         const int k = min(k0 + u * kSdThreads, end - 1);
@@ -160,7 +157,7 @@ sddmm_kernel(int64_t m, const int* __restrict__ Rst, const int* __restrict__ Col
 #pragma unroll
       for (int u = 0; u < kSdU; ++u) {
         const int k = k0 + u * kSdThreads;
-        if (k < end && c0 + k >= kb) dv[c0 + k] = gv[u] * xv[u];
+        if (ch.holds(k)) dv[ch.c0 + k] = gv[u] * xv[u];
       }
     }
     __syncthreads();  // the bitmap is read
