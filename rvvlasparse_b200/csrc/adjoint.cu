@@ -117,7 +117,7 @@ sddmm_kernel(int64_t m, const int* __restrict__ Rst, const int* __restrict__ Col
     __syncthreads();
     int earlier = 0;  // non-empty rows that start before the chunk
     if (t < rows) {
-      const int k = s_start[t] - ch.c0;
+      const int64_t k = s_start[t] - ch.c0;
       earlier = k < 0;
       if (k >= 0 && k < kSdChunk) atomicOr(&s_bits[k >> 5], 1u << (k & 31));
     }

@@ -2,6 +2,8 @@
 // and device code: which nonzeros a CTA's chunks read and write.
 #pragma once
 
+#include <cstdint>
+
 #ifdef __CUDACC__
 #define RVVLA_HD __host__ __device__
 #else
@@ -15,12 +17,14 @@ constexpr int kSdChunk = 4096;  // nonzeros per pass over the row-start bitmap
 // One chunk of a CTA's nonzeros [kb, ke): its slots k = 0 .. end() - 1 stand
 // for the nonzeros c0 + k.  Chunks start at multiples of 32, so the first one
 // may have slots before kb.
+// c0 has 64 bits: the step past the last chunk of 2^31 - 1 nonzeros leaves 32.
 struct SddmmChunk {
-  int c0, kb, ke;
-  RVVLA_HD int end() const { return ke - c0 < kSdChunk ? ke - c0 : kSdChunk; }
+  int64_t c0;
+  int kb, ke;
+  RVVLA_HD int end() const { return ke - c0 < kSdChunk ? (int)(ke - c0) : kSdChunk; }
   // the nonzero that slot k loads: slots outside [kb, ke) repeat its first or last
-  RVVLA_HD int load(int k) const {
-    const int j = c0 + (k < end() - 1 ? k : end() - 1);
+  RVVLA_HD int64_t load(int k) const {
+    const int64_t j = c0 + (k < end() - 1 ? k : end() - 1);
     return j > kb ? j : kb;
   }
   RVVLA_HD bool holds(int k) const { return k < end() && c0 + k >= kb; }

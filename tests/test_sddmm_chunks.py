@@ -47,3 +47,10 @@ def walk(tmp_path_factory):
 def test_loads_stay_in_the_rows_nonzeros(walk, kb):
     for n in [0, 1, 2, 31, 32, 33, 4095, 4096, 4097, 8192, 8193 + 31]:
         assert walk(kb, kb + n, 2048) == kb + n, n
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 4095, 4096, 5000, 10 ** 7 + 3])
+def test_largest_pattern(walk, n):
+    """2^31 - 1 nonzeros: the step past the last chunk does not fit 32 bits."""
+    end = 2 ** 31 - 1
+    assert walk(end - n, end, 2048) == end
