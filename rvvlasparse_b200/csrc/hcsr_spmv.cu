@@ -73,6 +73,7 @@
 
 #include "crs_merge.cuh"
 #include "crs_run.cuh"
+#include "hcsr_share.h"
 #include "rvvla_internal.cuh"
 
 namespace rvvla {
@@ -650,38 +651,38 @@ hcsr_spmv_kernel(int64_t R, int64_t C, int64_t m, int64_t nz, int64_t b_n, const
     }
 
     // ---- COO phase: rounds of kHRound nonzeros of the window's COO stream
-    // (this CTA's share: nonzeros [qlo, ntot) of it)
-    const int share = ((t_ent + split - 1) / split + 31) & ~31;
-    const int qlo = min(part * share, t_ent);
-    if (qlo < t_ent && share > 0) {
-      const int ncoo = t_coo, ntot = min(qlo + share, t_ent);
-      const int nrounds = (ntot - qlo + kHRound - 1) / kHRound;
+    // (this CTA's share: nonzeros [qs.lo, qs.hi) of it)
+    const HcsrShare qs = hcsr_share(t_ent, split, part);
+    if (qs.lo < qs.hi) {
+      const int ncoo = t_coo;
+      const unsigned ntot = (unsigned)qs.hi;
+      const int nrounds = qs.rounds(kHRound);
       HCooRaw<V> raw[kHU];
       auto coo_load = [&](int t) {
-        const int q00 = qlo + t * kHRound + warp * (kHU * 32);
+        const unsigned q00 = qs.first(t, kHRound, warp * (kHU * 32));
         // the block of the warp's first nonzero: the last that starts at or
         // before it, by two steps of 32 probes (list[0].cs is 0)
-        const int qs = min(q00, ntot - 1);
-        int ia = lane * kHProbe < ncoo && list[lane * kHProbe].cs <= qs;
+        const int qa = (int)min(q00, ntot - 1u);
+        int ia = lane * kHProbe < ncoo && list[lane * kHProbe].cs <= qa;
         ia = kHProbe * (__popc(__ballot_sync(0xffffffffu, ia)) - 1);
-        const bool le = lane < kHProbe && ia + lane < ncoo && list[ia + lane].cs <= qs;
+        const bool le = lane < kHProbe && ia + lane < ncoo && list[ia + lane].cs <= qa;
         ia += __popc(__ballot_sync(0xffffffffu, le)) - 1;
 #pragma unroll
         for (int u = 0; u < kHU; ++u) {
-          const int q0 = q00 + 32 * u;
+          const unsigned q0 = q00 + 32u * u;
           const int nxt = ia + 1 + lane;
-          const int d = nxt <= ncoo ? list[nxt].cs - q0 : 32;
+          const int d = nxt <= ncoo ? (int)((unsigned)list[nxt].cs - q0) : 32;
           const unsigned mask = __reduce_or_sync(0xffffffffu, (d >= 0 && d < 32) ? 1u << d : 0u);
           int blk = ia + __popc(mask & ((2u << lane) - 1u));
           blk = min(blk, ncoo - 1);
-          const int q = q0 + lane;
+          const unsigned q = q0 + lane;
           HCooRaw<V>& r = raw[u];
           r.ok = q < ntot;
           r.row = 0u;
           r.xoff = -1;
           if (r.ok) {
             const HBlk h = list[blk];
-            const int e = q - h.cs;
+            const int e = (int)q - h.cs;
             const int64_t k = (int64_t)h.bp + e;
             r.row = ld_stream(row_ptr + h.off + e, pf);
             r.col = (uint32_t)ld_stream(col_idx + k, pf);

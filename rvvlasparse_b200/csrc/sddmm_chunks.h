@@ -4,11 +4,7 @@
 
 #include <cstdint>
 
-#ifdef __CUDACC__
-#define RVVLA_HD __host__ __device__
-#else
-#define RVVLA_HD
-#endif
+#include "host_device.h"
 
 namespace rvvla {
 
