@@ -566,8 +566,9 @@ int rvvla_sddmm_values_f32(const rvvla_crs* A, const float* g, const float* x, f
  * X_i is n_i x k and Y_i is m_i x k, row-major, packed matrix after matrix
  * (matrix i starts at x_off[i] / y_off[i] elements). */
 typedef struct rvvla_batch {
-  int64_t count, k, x_len, y_len, ntiles;    /* ntiles: CSR tiles and SELL segments */
-  int32_t val_bytes, grid, block, sell_segs; /* sell_segs: the SELL segments among ntiles */
+  int64_t count, k, x_len, y_len, ntiles; /* ntiles: CSR tiles and SELL segments or parts */
+  int32_t val_bytes, grid, block;
+  int32_t sell_segs, sell_parts, reserved; /* the SELL segments and parts among ntiles (one of the two is 0) */
   const void* mats;   /* device table, one entry per matrix */
   const void* tiles;  /* device work list */
 } rvvla_batch;

@@ -75,7 +75,8 @@ class rvvla_transpose_owned(C.Structure):
 
 class rvvla_batch(C.Structure):
     _fields_ = [("count", i64), ("k", i64), ("x_len", i64), ("y_len", i64), ("ntiles", i64), ("val_bytes", i32),
-                ("grid", i32), ("block", i32), ("sell_segs", i32), ("mats", vp), ("tiles", vp)]
+                ("grid", i32), ("block", i32), ("sell_segs", i32), ("sell_parts", i32),
+                ("reserved", i32), ("mats", vp), ("tiles", vp)]
 
 
 class rvvla_batch_owned(C.Structure):

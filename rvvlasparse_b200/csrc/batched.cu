@@ -6,7 +6,7 @@
 // arrays) or as SELL-C-sigma (C = 32, built on the GPU and owned by the
 // plan).  All CSR matrices are one persistent launch over a list of tiles of
 // bounded work, all SELL matrices another over shares of slices; a plan of one
-// kind is one launch.
+// layout is one launch.
 //
 // Vectors: X_i is n_i x k and Y_i is m_i x k, row-major (the k values of one
 // row contiguous), packed one matrix after another; x_off/y_off give each
@@ -19,17 +19,22 @@
 // 64 MB; a 128-byte row takes 1.8 clocks), from L1 at three per clock, while
 // HBM brings 2.8 fp32 nonzeros per clock and SM.
 //
-// SELL kernel: one CTA per SM, a contiguous share of the slices per CTA, so
+// SELL kernels: one CTA per SM, a contiguous share of the slices per CTA, so
 // that all warps of an SM work on one matrix and its X rows stay in that SM's
 // L1 (k = 1: 240 us with one CTA of 32 warps per SM, 340 with two of 16 on
 // two shares, 410 with six of 8; a window of X in shared memory left L1 too
 // few lines for the loads in flight, 301).  For rows of 32 bytes and more X
 // does not fit L1 and balance counts more: each CTA takes four shorter pieces
 // from all over the batch (k = 8: 706 -> 602 us), and 16 warps keep eight row
-// loads per lane in flight (32 warps with four: 628).
-// 256 matrices of 1K to 65K rows (0.125G nonzeros, fp32, sigma 256), tiled
-// kernel before -> now: k = 1 468 -> 242, k = 4 1024 -> 515, k = 8 2602 -> 611,
-// k = 32 16738 -> 2223 us.
+// loads per lane in flight (32 warps with four: 628).  A CTA's share is divided
+// over its warps in parts, by load (batched_plan.h): cut matrix by matrix from
+// warp 0 on, a batch of matrices of fewer slices than warps kept a few warps
+// busy (20000 matrices of 32 rows, fp32: k = 1 387 us, 17 in parts; k = 8 524,
+// 42).  Large matrices are level cut that way too, and k = 1 takes 4 % less
+// time in such segments, whose loops run alike in all warps of a CTA.
+// 256 matrices of 1K to 65K rows (0.125G nonzeros, fp32, sigma 256), against
+// tiles of slices over all the CTAs that fit: k = 1 468 -> 242, k = 4 1024 ->
+// 510, k = 8 2602 -> 582, k = 32 16738 -> 1495 us.
 //
 // CSR kernel: a persistent grid of all the CTAs that fit walks the tiles with
 // a grid stride;
@@ -45,8 +50,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
+#include "batched_plan.h"
 #include "rvvla_internal.cuh"
 
 namespace rvvla {
@@ -77,14 +84,12 @@ struct BatchTile {
 // SELL: threads of the one CTA per SM (64 or 128 registers each), and the
 // pieces of the batch that a CTA takes.
 template <class T, int K> constexpr int kSThreads = K == 1 ? 1024 : 512;
-constexpr int kSWarpsMax = 32;
 constexpr int sell_pieces(int row_bytes) { return row_bytes >= 32 ? 4 : 1; }
-
-// A run of slices of one matrix: warp w of the CTA takes the slices
-// [first[w], first[w + 1]).
-struct BatchSeg {
-  int32_t mat, first[kSWarpsMax + 1];
-};
+// k = 1: segments as long as their busiest warp has at most this much more to
+// do than the parts' (256 matrices of 1K to 64K rows, fp32, 1.05: 243 us in
+// segments, 251 in parts; 400 of 6000 rows, 1.14: 92 and 79; 800 of 2000, 1.24:
+// 67 and 50; 20000 of 32, 26: 387 and 17)
+constexpr double kSegSlack = 1.12;
 
 template <class T> struct Vec16;
 template <> struct Vec16<float> { using type = float4; };
@@ -348,11 +353,35 @@ __device__ __forceinline__ void sell_slice(const BatchMat& A, int sl, const T* _
   }
 }
 
-// VEC: X and Y are 16-byte aligned (k > 1; for k = 1 there is one form).
+// The warp's parts.  VEC: X and Y are 16-byte aligned (k > 1; for k = 1 there
+// is one form).
 template <class T, int K, bool VEC>
 __global__ void __launch_bounds__(kSThreads<T, K>, 1)
-batched_sell_kernel(const BatchSeg* __restrict__ segs, const int* __restrict__ share,
+batched_sell_kernel(const int* __restrict__ share, const BatchPart* __restrict__ parts,
                     const BatchMat* __restrict__ mats, const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
+  int warp = threadIdx.x >> 5;
+  // a part's indexes are the same in all lanes; told so, the compiler keeps
+  // them in uniform registers, which k = 1 and 32 gain by (fp32, the batch
+  // above: 278 -> 251 and 1932 -> 1527 us) and k = 4 and 8 lose by (510 and 585
+  // -> 507 and 739; fp64 619 and 991 -> 620 and 1015)
+  if constexpr (K == 1 || K == 32) warp = __shfl_sync(0xffffffffu, warp, 0);
+  const int at = blockIdx.x * (kSThreads<T, K> / 32) + warp;
+  const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
+  const int p1 = share[at + 1];
+  for (int pi = share[at]; pi < p1; ++pi) {
+    const BatchPart p = parts[pi];
+    const BatchMat A = mats[p.mat];
+    const T* x = X + A.x_off;
+    for (int u = p.first; u < p.end; ++u) sell_slice<T, K, VEC>(A, u, x, Y, alpha, beta, pf, pl);
+  }
+}
+
+// The CTA's segments, k = 1.
+template <class T>
+__global__ void __launch_bounds__(kSThreads<T, 1>, 1)
+batched_seg_kernel(const int* __restrict__ share, const BatchSeg* __restrict__ segs,
+                   const BatchMat* __restrict__ mats, const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
+  static_assert(kSThreads<T, 1> == 32 * kSegWarps, "a segment is cut for the CTA's warps");
   const int warp = threadIdx.x >> 5;
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
   const int s1 = share[blockIdx.x + 1];
@@ -361,7 +390,7 @@ batched_sell_kernel(const BatchSeg* __restrict__ segs, const int* __restrict__ s
     const BatchMat& A = mats[sg.mat];
     const int u1 = sg.first[warp + 1];
     const T* x = X + A.x_off;
-    for (int u = sg.first[warp]; u < u1; ++u) sell_slice<T, K, VEC>(A, u, x, Y, alpha, beta, pf, pl);
+    for (int u = sg.first[warp]; u < u1; ++u) sell_slice<T, 1, true>(A, u, x, Y, alpha, beta, pf, pl);
   }
 }
 
@@ -415,16 +444,24 @@ template <class T, int K, bool VEC>
 int launch_k(const rvvla_batch* B, T alpha, const T* X, T beta, T* Y, cudaStream_t st) {
   const auto* mats = static_cast<const BatchMat*>(B->mats);
   const auto* tiles = static_cast<const BatchTile*>(B->tiles);
-  const int64_t ncsr = B->ntiles - B->sell_segs;
+  const int64_t ncsr = B->ntiles - B->sell_segs - B->sell_parts;
   if (ncsr > 0) {
     batched_kernel<T, K, VEC><<<B->grid, kBThreads, 0, st>>>(ncsr, tiles, mats, X, Y, alpha, beta);
     RVVLA_LAUNCHED("batched_kernel");
   }
-  if (B->sell_segs > 0) {
-    const auto* segs = reinterpret_cast<const BatchSeg*>(tiles + ncsr);
-    batched_sell_kernel<T, K, VEC><<<sm_count(), kSThreads<T, K>, 0, st>>>(
-        segs, reinterpret_cast<const int*>(segs + B->sell_segs), mats, X, Y, alpha, beta);
+  // after the tiles: the SELL work, then its shares
+  const auto* parts = reinterpret_cast<const BatchPart*>(tiles + ncsr);
+  const auto* segs = reinterpret_cast<const BatchSeg*>(parts + B->sell_parts);
+  const auto* share = reinterpret_cast<const int*>(segs + B->sell_segs);
+  if (B->sell_parts > 0) {
+    batched_sell_kernel<T, K, VEC><<<sm_count(), kSThreads<T, K>, 0, st>>>(share, parts, mats, X, Y, alpha, beta);
     RVVLA_LAUNCHED("batched_sell_kernel");
+  }
+  if constexpr (K == 1) {
+    if (B->sell_segs > 0) {
+      batched_seg_kernel<T><<<sm_count(), kSThreads<T, 1>, 0, st>>>(share, segs, mats, X, Y, alpha, beta);
+      RVVLA_LAUNCHED("batched_seg_kernel");
+    }
   }
   return RVVLA_OK;
 }
@@ -461,52 +498,6 @@ int resident_ctas(int k) {
                        : batched_kernel<T, 32, true>;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBThreads, 0) != cudaSuccess) per_sm = 1;
   return std::max(per_sm, 1);
-}
-
-struct SliceUnit {
-  int32_t mat, slice;
-  int64_t cost;  // columns, and a share for the slice itself
-};
-
-// Cuts the slices of all SELL matrices, in order, into grid * pieces runs of
-// equal cost, gives run r to CTA r mod grid, cuts each run by matrix into
-// segments and each segment by cost over the CTA's warps.  share[c] is CTA
-// c's first segment.
-void plan_slices(const std::vector<SliceUnit>& units, int grid, int pieces, int warps, std::vector<BatchSeg>& segs,
-                 std::vector<int32_t>& share) {
-  int64_t total = 0;
-  for (const SliceUnit& u : units) total += u.cost;
-  const int64_t runs = (int64_t)grid * pieces;
-  std::vector<std::vector<BatchSeg>> per((size_t)grid);
-  int64_t done = 0;
-  size_t u0 = 0;
-  for (int64_t r = 0; r < runs; ++r) {
-    const double until = (double)total * (double)(r + 1) / (double)runs;
-    size_t u1 = u0;
-    while (u1 < units.size() && (r + 1 == runs || (double)done + 0.5 * (double)units[u1].cost < until))
-      done += units[u1++].cost;
-    while (u0 < u1) {
-      BatchSeg sg = {};
-      sg.mat = units[u0].mat;
-      size_t ue = u0;
-      int64_t cost = 0, part = 0;
-      while (ue < u1 && units[ue].mat == sg.mat) cost += units[ue++].cost;
-      const int32_t end = units[ue - 1].slice + 1;
-      for (int w = 0; w < warps; ++w) {
-        while (u0 < ue && (double)part + 0.5 * (double)units[u0].cost < (double)cost * w / warps)
-          part += units[u0++].cost;
-        sg.first[w] = u0 < ue ? units[u0].slice : end;
-      }
-      for (int w = warps; w <= kSWarpsMax; ++w) sg.first[w] = end;
-      u0 = ue;
-      per[(size_t)(r % grid)].push_back(sg);
-    }
-  }
-  share.assign((size_t)grid + 1, 0);
-  for (int c = 0; c < grid; ++c) {
-    segs.insert(segs.end(), per[(size_t)c].begin(), per[(size_t)c].end());
-    share[(size_t)c + 1] = (int32_t)segs.size();
-  }
 }
 
 // Times one plan: one warm-up launch, then the best of three (CUDA events on
@@ -670,12 +661,15 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
   h.val_bytes = val_bytes;
   h.x_len = out->x_off[count];
   h.y_len = out->y_off[count];
-  std::vector<BatchSeg> segs;
-  std::vector<int32_t> share;
-  plan_slices(slices, sm_count(), sell_pieces(k * val_bytes), (k == 1 ? kSThreads<float, 1> : kSThreads<float, 8>) / 32,
-              segs, share);
-  h.sell_segs = (int32_t)segs.size();
-  h.ntiles = (int64_t)(tiles.size() + segs.size());
+  const int warps = (k == 1 ? kSThreads<float, 1> : kSThreads<float, 8>) / 32, pieces = sell_pieces(k * val_bytes);
+  SlicePlan sp = plan_parts(slices, sm_count(), pieces, warps);
+  if (k == 1) {
+    SlicePlan sg = plan_segments(slices, sm_count(), pieces);
+    if ((double)sg.busiest <= kSegSlack * (double)sp.busiest) sp = std::move(sg);
+  }
+  h.sell_segs = (int32_t)sp.segs.size();
+  h.sell_parts = (int32_t)sp.parts.size();
+  h.ntiles = (int64_t)tiles.size() + h.sell_segs + h.sell_parts;
   auto fail_cuda = [&](cudaError_t e, const char* where) {
     const int r = cuda_fail(e, where);
     std::string keep = rvvla_last_error();
@@ -686,24 +680,23 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
   cudaError_t e;
   if ((e = cudaMalloc(&out->mats, std::max<size_t>(tab.size(), 1) * sizeof(BatchMat))) != cudaSuccess)
     return fail_cuda(e, "cudaMalloc(mats)");
-  // the CSR tiles, the SELL segments and the CTAs' shares of them
-  const size_t tile_bytes = tiles.size() * sizeof(BatchTile), seg_bytes = segs.size() * sizeof(BatchSeg);
-  const size_t share_bytes = share.size() * sizeof(int32_t);
-  if ((e = cudaMalloc(&out->tiles, tile_bytes + seg_bytes + share_bytes)) != cudaSuccess)
-    return fail_cuda(e, "cudaMalloc(tiles)");
+  // the CSR tiles, the SELL parts, the SELL segments, their shares
+  const std::pair<const void*, size_t> lists[] = {{tiles.data(), tiles.size() * sizeof(BatchTile)},
+                                                  {sp.parts.data(), sp.parts.size() * sizeof(BatchPart)},
+                                                  {sp.segs.data(), sp.segs.size() * sizeof(BatchSeg)},
+                                                  {sp.share.data(), sp.share.size() * sizeof(int32_t)}};
+  size_t bytes = 0;
+  for (const auto& l : lists) bytes += l.second;
+  if ((e = cudaMalloc(&out->tiles, bytes)) != cudaSuccess) return fail_cuda(e, "cudaMalloc(tiles)");
   if (!tab.empty() &&
       (e = cudaMemcpyAsync(out->mats, tab.data(), tab.size() * sizeof(BatchMat), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return fail_cuda(e, "cudaMemcpyAsync(mats)");
-  char* d_tiles = static_cast<char*>(out->tiles);
-  if (!tiles.empty() &&
-      (e = cudaMemcpyAsync(d_tiles, tiles.data(), tile_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
-    return fail_cuda(e, "cudaMemcpyAsync(tiles)");
-  if (!segs.empty() &&
-      (e = cudaMemcpyAsync(d_tiles + tile_bytes, segs.data(), seg_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
-    return fail_cuda(e, "cudaMemcpyAsync(segments)");
-  if ((e = cudaMemcpyAsync(d_tiles + tile_bytes + seg_bytes, share.data(), share_bytes, cudaMemcpyHostToDevice,
-                           st)) != cudaSuccess)
-    return fail_cuda(e, "cudaMemcpyAsync(shares)");
+  char* to = static_cast<char*>(out->tiles);
+  for (const auto& l : lists) {
+    if (l.second && (e = cudaMemcpyAsync(to, l.first, l.second, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+      return fail_cuda(e, "cudaMemcpyAsync(tiles)");
+    to += l.second;
+  }
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, "cudaStreamSynchronize");
   // persistent grid of the CSR kernel: every SM filled with as many CTAs as fit
   const int per_sm = (val_bytes == 8) ? resident_ctas<double>(k) : resident_ctas<float>(k);
@@ -729,7 +722,7 @@ int rvvla_batched_graph(const rvvla_batch* B, double alpha, const void* X, doubl
   cudaStream_t st = as_stream(stream);
   if (!st) return fail(RVVLA_ERR_INVALID_ARG, "batched_graph: capture needs a non-default stream");
   auto* g = new BatchGraph();
-  g->kernels = (B->ntiles > B->sell_segs ? 1 : 0) + (B->sell_segs > 0 ? 1 : 0);
+  g->kernels = (B->ntiles > B->sell_segs + B->sell_parts ? 1 : 0) + (B->sell_segs + B->sell_parts > 0 ? 1 : 0);
   const cudaError_t eb = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (eb != cudaSuccess) {
     delete g;
