@@ -28,8 +28,8 @@
  *     names, same meaning), with device pointers.
  *   - Entry points that need temporary device memory obtain it stream-ordered
  *     on `stream`: products and solvers from a memory pool of the library's own
- *     (the ordinary fp64 CSR5 product, requests above 256 MB and the builders:
- *     from the device's default pool).  Between calls that pool keeps at most
+ *     (the ordinary fp64 CSR5 product, requests above 256 MB and the builders, but
+ *     for SELL's of up to 2^20 rows: from the device's default pool).  Between calls that pool keeps at most
  *     256 MB per device; rvvla_trim_scratch() gives it back.
  */
 #ifndef RVVLA_H

@@ -593,16 +593,16 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
     out->x_off[i + 1] = out->x_off[i] + A.n * k;
     out->y_off[i + 1] = out->y_off[i] + A.m * k;
     if (A.m == 0) continue;
-    Rst.resize((size_t)A.m + 1);
-    if (cudaMemcpyAsync(Rst.data(), A.Rst, (A.m + 1) * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
-      rc = fail(RVVLA_ERR_CUDA, "batched_plan: reading row pointers failed");
-      break;
-    }
     const int md = mode ? mode[i] : 0;
     const double avg = (double)A.nz / (double)A.m;
     if (md == 0) {
       b.mode = 0;
+      Rst.resize((size_t)A.m + 1);  // the tiles are cut on the host
+      if (cudaMemcpyAsync(Rst.data(), A.Rst, (A.m + 1) * sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+          cudaStreamSynchronize(st) != cudaSuccess) {
+        rc = fail(RVVLA_ERR_CUDA, "batched_plan: reading row pointers failed");
+        break;
+      }
       const int tpr = (param && param[i] > 0) ? param[i] : default_tpr(avg);
       if (tpr > 32 || (tpr & (tpr - 1))) {
         rc = fail(RVVLA_ERR_INVALID_ARG, "batched_plan: threads per row must be a power of two <= 32");

@@ -70,7 +70,8 @@ cudaMemPool_t scratch_pool();
 // 4M power-law rows, first call on a new matrix: 883 us, 406 us with the kept
 // pool; a first CG solve on 4M rows 8.7 -> 6.0 ms).  Builders stay away from
 // it: the LAV builder's buffers, trimmed to the limit at each of its
-// synchronisations, took 118 ms instead of 31.
+// synchronisations, took 118 ms instead of 31; the SELL builder takes its
+// buffers there where they are small (a batch's matrices).
 constexpr uint64_t kScratchKeep = 256ull << 20;  // a solve on 8M rows in fp64 fits
 struct Scratch {
   void* p = nullptr;

@@ -97,7 +97,7 @@ int exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t 
   }
   const int64_t nchunks = (n + kChunk - 1) / kChunk;
   Scratch sc;
-  RVVLA_CUDA(sc.alloc((size_t)(nchunks + 1) * sizeof(int64_t), st));
+  RVVLA_CUDA(sc.alloc_kept((size_t)(nchunks + 1) * sizeof(int64_t), st));
   chunk_sum_kernel<<<(unsigned)nchunks, kScanThreads, 0, st>>>(in, n, sc.as<int64_t>());
   RVVLA_LAUNCHED("chunk_sum_kernel");
   sums_scan_kernel<<<1, 1024, 0, st>>>(sc.as<int64_t>(), nchunks);

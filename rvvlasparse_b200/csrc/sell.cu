@@ -322,9 +322,13 @@ int sell_build_impl(const rvvla_crs* src, int vb, int64_t C, int64_t sigma, rvvl
   int64_t total = 0;
   if (m > 0) {
     Scratch s_key, s_key2, s_idx, s_tmp, s_area, s_off;
-    RVVLA_CUDA(s_key.alloc((size_t)m * sizeof(uint64_t), st));
-    RVVLA_CUDA(s_key2.alloc((size_t)m * sizeof(uint64_t), st));
-    RVVLA_CUDA(s_idx.alloc((size_t)m * sizeof(uint32_t), st));
+    // small matrices' buffers (under 64 MB) from the kept pool: the default pool
+    // gives them back at each build's synchronisations, and a batch builds many
+    // (256 matrices of 1K to 64K rows: 246 ms, 131 from the kept pool)
+    auto take = [&](Scratch& s, size_t bytes) { return m <= (1 << 20) ? s.alloc_kept(bytes, st) : s.alloc(bytes, st); };
+    RVVLA_CUDA(take(s_key, (size_t)m * sizeof(uint64_t)));
+    RVVLA_CUDA(take(s_key2, (size_t)m * sizeof(uint64_t)));
+    RVVLA_CUDA(take(s_idx, (size_t)m * sizeof(uint32_t)));
     sell_keys_kernel<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(m, sigma, src->Rst, s_key.as<uint64_t>(),
                                                                    s_idx.as<uint32_t>());
     RVVLA_LAUNCHED("sell_keys_kernel");
@@ -334,12 +338,12 @@ int sell_build_impl(const rvvla_crs* src, int vb, int64_t C, int64_t sigma, rvvl
     size_t tmp_bytes = 0;
     RVVLA_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, s_key.as<uint64_t>(), s_key2.as<uint64_t>(),
                                                s_idx.as<uint32_t>(), out->vPerm, (int)m, 0, end_bit, st));
-    RVVLA_CUDA(s_tmp.alloc(tmp_bytes, st));
+    RVVLA_CUDA(take(s_tmp, tmp_bytes));
     RVVLA_CUDA(cub::DeviceRadixSort::SortPairs(s_tmp.p, tmp_bytes, s_key.as<uint64_t>(), s_key2.as<uint64_t>(),
                                                s_idx.as<uint32_t>(), out->vPerm, (int)m, 0, end_bit, st));
     count_launch(3);
-    RVVLA_CUDA(s_area.alloc((size_t)(cnt_b + 1) * sizeof(int64_t), st));
-    RVVLA_CUDA(s_off.alloc((size_t)(cnt_b + 1) * sizeof(int64_t), st));
+    RVVLA_CUDA(take(s_area, (size_t)(cnt_b + 1) * sizeof(int64_t)));
+    RVVLA_CUDA(take(s_off, (size_t)(cnt_b + 1) * sizeof(int64_t)));
     sell_slices_kernel<<<(unsigned)((cnt_b + 255) / 256), 256, 0, st>>>(m, C, cnt_b, src->Rst, out->vPerm, out->vCl,
                                                                          out->vBs, out->vSBs, s_area.as<int64_t>());
     RVVLA_LAUNCHED("sell_slices_kernel");
