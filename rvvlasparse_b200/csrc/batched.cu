@@ -43,8 +43,12 @@
 //   k > 1   the tile's columns and values (at most 2048 nonzeros) are staged in
 //           shared memory with one coalesced pass; spr groups of G lanes per
 //           row read them from there and gather X, shuffle reduction over the
-//           groups (same batch: k = 4 918 -> 755, k = 8 1293 -> 947, k = 32 3159 ->
-//           1836 us against k lanes of one value each).
+//           groups (same batch: k = 4 918 -> 755, k = 8 1293 -> 930, k = 32 3159 ->
+//           1767 us against k lanes of one value each).  Each group keeps two
+//           sums and adds four products at a time to one of them in turn, so
+//           that a row's error is no larger than that of eight sums (2 and
+//           1000 nonzeros a row, fp32, relative error: 3.6e-7 with two sums
+//           that take the products one by one, 1.8e-7 with eight, 8.5e-8 now).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -74,11 +78,11 @@ struct BatchMat {
   const uint32_t* sPerm;
   const void* sVal;
   int64_t x_off, y_off;
-  int32_t m, n, mode, tpr;  // tpr: lane groups per row (CSR)
+  int32_t m, n, mode, tpr;  // tpr: lanes per row (CSR, k = 1)
 };
 
 struct BatchTile {
-  int32_t mat, first, count, pad;
+  int32_t mat, first, count, spr;  // spr: lane groups per row, k > 1
 };
 
 // SELL: threads of the one CTA per SM (64 or 128 registers each), and the
@@ -203,7 +207,7 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
                        T* __restrict__ s_val, const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
   using XR = XRows<T, K, VEC>;
   constexpr int VPL = XR::VPL, G = XR::G, U = 4;
-  const int spr = A.tpr, lanes = G * spr, nslots = kBThreads / lanes;
+  const int spr = t.spr, lanes = G * spr, nslots = kBThreads / lanes;
   const int part = threadIdx.x % G, slot = (threadIdx.x / G) % spr, sub = threadIdx.x / lanes;
   const T* __restrict__ x = X + A.x_off + part * VPL;
   const T* __restrict__ val = static_cast<const T*>(A.Val);
@@ -224,15 +228,26 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
   for (int it = 0; it < iters; ++it) {
     const int rr = it * nslots + sub;
     const bool valid = rr < t.count;
+    // the steps' sums go to two accumulators in turn: no chain of roundings is
+    // longer than an eighth of the row and a few
     T acc[2][VPL];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) acc[0][i] = acc[1][i] = T(0);
+    auto add_step = [&](const T (&t)[VPL]) {
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        const T a = acc[0][i] + t[i];
+        acc[0][i] = acc[1][i];
+        acc[1][i] = a;
+      }
+    };
     if (valid) {
       const int e = srst[rr + 1] - b0;
       int j = srst[rr] - b0 + slot;
       // rows of 128 bytes and more: whole steps, then one nonzero at a time (a
       // repeated row would cost as much as a new one); narrower ones: idle
       // loads of the last step repeat its first entry
+#pragma unroll(G >= 8 ? 2 : 1)
       for (; G >= 8 ? j + (U - 1) * spr < e : j < e; j += U * spr) {
         T v[U];
         alignas(16) T xv[U][VPL];
@@ -243,21 +258,29 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
           v[u] = staged ? s_val[k] : val[b0 + k];
           gather_n<T, VPL, VEC>(x + (int64_t)c * K, xv[u], pl);
         }
+        T t[VPL];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int i = 0; i < VPL; ++i) t[i] = v[0] * xv[0][i];
+#pragma unroll
+        for (int u = 1; u < U; ++u)
           if (G >= 8 || j + u * spr < e) {
 #pragma unroll
-            for (int i = 0; i < VPL; ++i) acc[u & 1][i] += v[u] * xv[u][i];
+            for (int i = 0; i < VPL; ++i) t[i] += v[u] * xv[u][i];
           }
+        add_step(t);
       }
+      T t[VPL];
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) t[i] = T(0);
       for (; G >= 8 && j < e; j += spr) {
         const int c = staged ? s_col[j] : A.Col[b0 + j];
         const T v = staged ? s_val[j] : val[b0 + j];
         alignas(16) T xv[VPL];
         gather_n<T, VPL, VEC>(x + (int64_t)c * K, xv, pl);
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) acc[0][i] += v * xv[i];
+        for (int i = 0; i < VPL; ++i) t[i] += v * xv[i];
       }
+      if (G >= 8) add_step(t);
     }
     alignas(16) T s[VPL];
 #pragma unroll
@@ -394,8 +417,10 @@ batched_seg_kernel(const int* __restrict__ share, const BatchSeg* __restrict__ s
   }
 }
 
+// Five CTAs per SM in fp64 (k = 4: 1232 us for the batch above with the four
+// that the registers allow otherwise, 1120 with five and a little spilled).
 template <class T, int K, bool VEC>
-__global__ void __launch_bounds__(kBThreads)
+__global__ void __launch_bounds__(kBThreads, K > 1 && sizeof(T) == 8 ? 5 : 0)
 batched_kernel(int64_t ntiles, const BatchTile* __restrict__ tiles, const BatchMat* __restrict__ mats,
                const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
   // per tile: the matrix entry and the tile's row pointers are copied to
@@ -433,10 +458,12 @@ int lanes_nz(int k, int vb) { return k == 1 ? 1 : k * vb / 16; }
 
 // Lane groups per CSR row for k > 1: at least eight nonzeros per group (fewer
 // leave more of the four loads per lane and step idle: k = 4 / 8 fp32, the
-// batch above: 907 / 1168 us with two per group, 759 / 1010 with eight).
-int default_spr(double avg, int lanes) {
+// batch above: 907 / 1168 us with two per group, 759 / 1010 with eight), but in
+// a tile with a long row enough for at most 32 nonzeros per group, which bounds
+// both the time that row takes and the roundings in its sums.
+int default_spr(double avg, int64_t longest, int lanes) {
   int t = 1;
-  while (2 * t * lanes <= 32 && 16 * t <= avg) t <<= 1;
+  while (2 * t * lanes <= 32 && (16 * t <= avg || 32 * t < longest)) t <<= 1;
   return t;
 }
 
@@ -608,22 +635,23 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
         rc = fail(RVVLA_ERR_INVALID_ARG, "batched_plan: threads per row must be a power of two <= 32");
         break;
       }
-      b.tpr = (k == 1) ? tpr : default_spr(avg, lanes_nz(k, val_bytes));
-      const int lanes_row = (k == 1) ? tpr : b.tpr * lanes_nz(k, val_bytes);
+      b.tpr = tpr;
+      const int lanes = lanes_nz(k, val_bytes), lanes_row = (k == 1) ? tpr : default_spr(avg, 0, lanes) * lanes;
       // tiles of whole rows: k = 1 at most kTileWork nonzeros and 8 row
       // passes of the CTA; k > 1 at most the staged nonzeros and 32 passes
       const int64_t max_rows = std::min<int64_t>((int64_t)(kBThreads / lanes_row) * (k == 1 ? 8 : 32), kTileRowsMax);
       const int64_t max_work = k == 1 ? kTileWork : kStageNnz;
       int64_t r0 = 0;
       while (r0 < A.m) {
-        int64_t r1 = r0, work = 0;
+        int64_t r1 = r0, work = 0, longest = 0;
         while (r1 < A.m && r1 - r0 < max_rows) {
           const int64_t wr = (int64_t)Rst[(size_t)r1 + 1] - Rst[(size_t)r1] + (k == 1 ? 1 : 0);
           if (r1 > r0 && work + wr > max_work) break;
           work += wr;
+          longest = std::max(longest, wr);
           ++r1;
         }
-        tiles.push_back({(int32_t)i, (int32_t)r0, (int32_t)(r1 - r0), 0});
+        tiles.push_back({(int32_t)i, (int32_t)r0, (int32_t)(r1 - r0), k == 1 ? tpr : default_spr(avg, longest, lanes)});
         r0 = r1;
       }
     } else if (md == 1) {
