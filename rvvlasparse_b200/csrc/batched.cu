@@ -293,18 +293,24 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
   }
 }
 
-// One SELL slice by one warp: U columns of values and column indices are
-// loaded, then X rows, UX columns at a time.  P partial sums per row, as many
-// as the registers allow.
+// One SELL slice by one warp.  U columns of values and column indices are
+// loaded, then X rows, UX columns of GX rows per lane group at a time.  For k > 1
+// four columns' products of a row make a block, and the blocks' sums go to P
+// accumulators in turn, which makes the chains of roundings about as short as in
+// CSR's sums (error of the batch above, fp32, k = 8: 7.34e-8 with four sums that
+// took a product each, 6.84e-8 in blocks; fp64, k = 8, 1061 -> 888 us with
+// it).  Rows of 256 bytes leave no registers for that (5830 us against 3815) and
+// take one column of all rows at a time into one sum.  For k = 1 the products
+// go to four sums.
 template <class T, int K, bool VEC>
 __device__ __forceinline__ void sell_slice(const BatchMat& A, int sl, const T* __restrict__ x, T* __restrict__ Y,
                                            T alpha, T beta, uint64_t pf, uint64_t pl) {
   using XR = XRows<T, K, VEC>;
   constexpr int VPL = XR::VPL, G = XR::G;
-  constexpr int P = K * sizeof(T) >= 128 ? 1 : K * sizeof(T) == 64 ? 2 : 4;
-  constexpr int U = G == 1 ? 8 : 4, XL = 8;  // columns, and X loads per lane, in flight
-  constexpr int UX = G == 1 ? U : XL / G > 0 ? XL / G : 1;
-  constexpr int GB = G < XL ? G : XL;
+  constexpr bool BLOCKS = K > 1 && K * sizeof(T) < 256;
+  constexpr int U = G <= 4 ? 8 : 4;
+  constexpr int P = K == 1 ? 4 : BLOCKS ? U / 4 : 1;
+  constexpr int UX = K == 1 ? U : BLOCKS ? 4 : 1, GX = G == 1 ? 1 : BLOCKS ? 2 : 8;
   constexpr int RS = 32 / G;  // rows per step
   const int lane = threadIdx.x & 31, part = lane % G;
   const T* __restrict__ val = static_cast<const T*>(A.sVal);
@@ -331,15 +337,15 @@ __device__ __forceinline__ void sell_slice(const BatchMat& A, int sl, const T* _
     }
 #pragma unroll
     for (int u0 = 0; u0 < U; u0 += UX) {
-      if (u0 > 0 && j + u0 >= w) break;  // warp-uniform
+      if (G > 1 && u0 > 0 && j + u0 >= w) break;  // warp-uniform
 #pragma unroll
-      for (int g0 = 0; g0 < G; g0 += GB) {
-        alignas(16) T xv[UX][GB][VPL];
-        T vv[UX][GB];
+      for (int g0 = 0; g0 < G; g0 += GX) {
+        alignas(16) T xv[UX][GX][VPL];
+        T vv[UX][GX];
 #pragma unroll
         for (int u = 0; u < UX; ++u)
 #pragma unroll
-          for (int g = 0; g < GB; ++g) {
+          for (int g = 0; g < GX; ++g) {
             if constexpr (G == 1) {
               vv[u][g] = v[u0 + u];
               gather_n<T, VPL, VEC>(x + (int64_t)c[u0 + u] * K, xv[u][g], pl);
@@ -351,12 +357,20 @@ __device__ __forceinline__ void sell_slice(const BatchMat& A, int sl, const T* _
             }
           }
 #pragma unroll
-        for (int u = 0; u < UX; ++u)
-          if (j + u0 + u < w) {
+        for (int g = 0; g < GX; ++g)
 #pragma unroll
-            for (int g = 0; g < GB; ++g)
+          for (int i = 0; i < VPL; ++i) {
+            if constexpr (BLOCKS) {
+              T t = vv[0][g] * xv[0][g][i];
 #pragma unroll
-              for (int i = 0; i < VPL; ++i) acc[(u0 + u) % P][g0 + g][i] += vv[u][g] * xv[u][g][i];
+              for (int u = 1; u < UX; ++u)
+                if (j + u0 + u < w) t += vv[u][g] * xv[u][g][i];
+              if (G > 1 || j + u0 < w) acc[u0 / 4][g0 + g][i] += t;
+            } else {
+#pragma unroll
+              for (int u = 0; u < UX; ++u)
+                if (j + u0 + u < w) acc[(u0 + u) % P][g0 + g][i] += vv[u][g] * xv[u][g][i];
+            }
           }
       }
     }
