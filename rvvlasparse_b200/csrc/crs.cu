@@ -164,9 +164,8 @@ int crs_plan_launch(int64_t m, int64_t nz, const int32_t* Rst, int ipt, int32_t*
 // the blocks' sums, in block order, into *dot.  `ticket` is 0 before and after.
 template <class X, class CT>
 __global__ void __launch_bounds__(256)
-crs_dot_fixup_kernel(int nw, const int* __restrict__ carry_row, const CT* __restrict__ carry_val, X* __restrict__ y,
-                     X alpha, X beta, const int* __restrict__ row_map, const CT* __restrict__ part,
-                     double* __restrict__ sums, unsigned* __restrict__ ticket, double* __restrict__ dot) {
+crs_dot_fixup_kernel(int nw, const int* carry_row, const CT* carry_val, X* y, X alpha, X beta,
+                     const int* __restrict__ row_map, const CT* part, double* sums, unsigned* ticket, double* dot) {
   __shared__ double sh[256];
   __shared__ bool last;
   const int t = threadIdx.x;

@@ -92,7 +92,8 @@ __device__ __forceinline__ void run_idx(const int* p, int (&v)[kRunLane], uint64
 // every row piece v that leaves the kernel (stored, or handed on as a carry)
 // also adds x[row] * v to the warp's partial dot_part[w], so the warps'
 // partials sum to x^T (A x) without a second pass over y (the solvers'
-// fused SpMV-dot; square A).
+// fused SpMV-dot; square A; x, the solver's p, is what the kernel before in the
+// chain wrote).
 // TPB: threads per CTA (the warps do not cooperate).
 template <class V, class X, class Ac, class CT, int TPB, bool VEC, bool PERM = false, bool DOT = false>
 __global__ void __launch_bounds__(TPB)
@@ -117,7 +118,7 @@ crs_run_kernel(int m, int nnz, int E, int nwarps, const int* __restrict__ rst, c
   auto yrow = [&](int r) { return row_map ? row_map[r] : r; };
   CT dotv = CT(0);  // DOT: this lane's share of x^T (A x)
   auto dot_add = [&](int r, CT v) {
-    if constexpr (DOT) dotv += (CT)x[yrow(r)] * v;
+    if constexpr (DOT) dotv += (CT)ld_chain(x + yrow(r), pl) * v;
   };
   // closes the open row (complete): the warp's first row may have begun in
   // an earlier warp, then it becomes a carry instead of a store
@@ -157,7 +158,7 @@ crs_run_kernel(int m, int nnz, int E, int nwarps, const int* __restrict__ rst, c
     using PT = decltype(vmul(V(), X()));
     PT p[kRunLane];
 #pragma unroll
-    for (int i = 0; i < kRunLane; ++i) p[i] = vmul(vv[i], ld_keep(x + cidx[i], pl));
+    for (int i = 0; i < kRunLane; ++i) p[i] = vmul(vv[i], DOT ? ld_chain(x + cidx[i], pl) : ld_keep(x + cidx[i], pl));
     unsigned fl = nv > 0 ? (bits[a >> 5] >> (a & 31)) & ((1u << nv) - 1u) : 0u;
     // a mark on the chunk's first nonzero closes the open row before it
     const bool start0 = __shfl_sync(0xffffffffu, fl & 1u, 0) != 0u;

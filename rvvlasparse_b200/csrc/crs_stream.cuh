@@ -169,9 +169,8 @@ crs_stream_kernel(int m, int nnz, int E, int nwarps, const int* __restrict__ Rst
 // Rows that cross warp boundaries: every piece is a carry (no warp wrote the
 // row), so the run of equal rows is summed in warp order and written once.
 template <class X, class CT>
-__device__ __forceinline__ void crs_fixup_slot(int t, int nslots, const int* __restrict__ carry_row,
-                                               const CT* __restrict__ carry_val, X* __restrict__ y, X alpha, X beta,
-                                               const int* __restrict__ row_map) {
+__device__ __forceinline__ void crs_fixup_slot(int t, int nslots, const int* carry_row, const CT* carry_val, X* y, X alpha,
+                                               X beta, const int* __restrict__ row_map) {
   if (t >= nslots) return;
   const int r = carry_row[t];
   if (r < 0) return;
@@ -191,8 +190,7 @@ __device__ __forceinline__ void crs_fixup_slot(int t, int nslots, const int* __r
 }
 
 template <class X, class CT>
-__global__ void crs_stream_fixup_kernel(int nslots, const int* __restrict__ carry_row,
-                                        const CT* __restrict__ carry_val, X* __restrict__ y, X alpha, X beta,
+__global__ void crs_stream_fixup_kernel(int nslots, const int* carry_row, const CT* carry_val, X* y, X alpha, X beta,
                                         const int* __restrict__ row_map) {
   grid_chain();
   crs_fixup_slot((int)(blockIdx.x * blockDim.x + threadIdx.x), nslots, carry_row, carry_val, y, alpha, beta, row_map);

@@ -581,8 +581,7 @@ csr5_spmv_generic_kernel(int64_t nfull, int tiles_per_warp, int sigma, int by, i
 // Calibrator merge in warp order (:318-335): a run of warps continuing one
 // row is summed first, then added once.
 template <class X, class CT>
-__global__ void csr5_calibrate_kernel(int64_t nwarps, const int* __restrict__ cal_row, const CT* __restrict__ cal,
-                                      X* __restrict__ y, X alpha) {
+__global__ void csr5_calibrate_kernel(int64_t nwarps, const int* cal_row, const CT* cal, X* y, X alpha) {
   grid_chain();
   const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nwarps) return;
@@ -600,7 +599,7 @@ __global__ void csr5_calibrate_kernel(int64_t nwarps, const int* __restrict__ ca
 template <class V, class X, class Ac, class CT>
 __global__ void csr5_tail_kernel(int64_t m, int64_t tail_row, int64_t tail_start, const int* __restrict__ Rst,
                                  const uint32_t* __restrict__ colidx, const V* __restrict__ vals,
-                                 const X* __restrict__ x, X* __restrict__ y, X alpha, X beta) {
+                                 const X* __restrict__ x, X* y, X alpha, X beta) {
   using Ops = LaneOps<V, X, Ac, CT>;
   grid_chain();
   const int64_t r = tail_row + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -202,7 +202,7 @@ template <class V, class X, class CT>
 __global__ void __launch_bounds__(256, sizeof(V) >= 8 ? 3 : 4)
 cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ vals,
                 const uint32_t* __restrict__ cols, const int* __restrict__ rec, const int* __restrict__ wb,
-                const X* __restrict__ x, X* __restrict__ y, X alpha) {
+                const X* __restrict__ x, X* y, X alpha) {
   constexpr int kCvrU = kCvrBatch;
   constexpr int kRanges = 8 / kCvrSplit;  // ranges per CTA
   __shared__ int s_row[8][kCvrU][kS];

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(256)
 lav_fused_kernel(int64_t nseg, int64_t cc, int64_t m, int64_t n, int64_t nlong, const int* __restrict__ co,
                  const int* __restrict__ cf, const uint64_t* __restrict__ sp, const uint16_t* __restrict__ mk,
                  const V* __restrict__ val, const uint32_t* __restrict__ col, const uint8_t* __restrict__ los,
-                 const uint32_t* __restrict__ row_order, const X* __restrict__ x, X* __restrict__ y, X alpha) {
+                 const uint32_t* __restrict__ row_order, const X* __restrict__ x, X* y, X alpha) {
   static_assert(32 % L == 0, "a chunk must not straddle warps");
   constexpr int G = 256 / L;
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();

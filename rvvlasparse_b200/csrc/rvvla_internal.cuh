@@ -123,6 +123,11 @@ inline cudaError_t launch_chained(void (*kernel)(P...), unsigned blocks, unsigne
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// What the kernels before it in the chain write, a chained kernel reads through
+// ordinary loads from pointers without __restrict__, or ld_chain: ld.global.nc
+// and a restrict argument promise data that nothing writes while the kernel
+// runs, and it runs from before its wait on, so that either may be read early.
+//
 // By every CTA that does any work: chain_open lets the stream's next chained
 // kernel start once all CTAs have come here, chain_wait waits until the
 // previous kernel is complete and its writes are visible (at once in a kernel
@@ -138,8 +143,9 @@ __device__ __forceinline__ void grid_chain() {
 // Streaming operands (values, indices) are read once: evict-first in L2 and
 // no L1 allocation.  The gathered vector x is re-read across the whole matrix:
 // evict-last keeps it resident in the 126 MB L2.  The asm statements are not
-// volatile: they are pure reads of data the kernels never write, so the
-// compiler may hoist and batch them to keep many loads in flight.
+// volatile: they are pure reads of data that neither the kernel nor one that it
+// is chained to writes, so the compiler may hoist and batch them to keep many
+// loads in flight.
 __device__ __forceinline__ uint64_t policy_evict_first() {
   uint64_t p;
   asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -199,6 +205,19 @@ template <> __device__ __forceinline__ double ld_keep<double>(const double* p, u
 template <> __device__ __forceinline__ float ld_keep<float>(const float* p, uint64_t pol) {
   float v;
   asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  return v;
+}
+
+// The gathered vector where the kernel before in the chain wrote it (see
+// launch_chained): a coherent load that stays behind the wait.
+__device__ __forceinline__ double ld_chain(const double* p, uint64_t pol) {
+  double v;
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_chain(const float* p, uint64_t pol) {
+  float v;
+  asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol) : "memory");
   return v;
 }
 

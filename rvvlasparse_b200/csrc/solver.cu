@@ -102,8 +102,8 @@ __device__ __forceinline__ double cg_alpha(const CgScalars* s, int cur) {
 // r -= alpha q and the new r.r: the block that finishes last adds the blocks'
 // partials in a fixed order.
 template <class T>
-__global__ void __launch_bounds__(kUpdThreads) cg_update_kernel(int64_t n, T* __restrict__ r, const T* __restrict__ q,
-                                                                CgScalars* s, int cur, double* part) {
+__global__ void __launch_bounds__(kUpdThreads) cg_update_kernel(int64_t n, T* r, const T* q, CgScalars* s, int cur,
+                                                                double* part) {
   __shared__ bool last;
   grid_chain();
   // r and q start 16-byte aligned: 16 bytes a thread, two loads of each in flight
@@ -206,16 +206,15 @@ int spmv_dot_impl(const rvvla_crs* A, const T* x, T* y, T* dot, cudaStream_t st)
 
 // x += alpha p, p = r + beta p: the x update shares the read of p.
 template <class T>
-__global__ void cg_xp_kernel(int64_t n, T* __restrict__ x, T* __restrict__ p, const T* __restrict__ r,
-                             const CgScalars* s, int cur) {
+__global__ void cg_xp_kernel(int64_t n, T* x, T* p, const T* r, const CgScalars* s, int cur) {
   grid_chain();
   const T alpha = (T)cg_alpha(s, cur);
   const T beta = (T)(s->rr[cur] != 0.0 ? s->rr[cur ^ 1] / s->rr[cur] : 0.0);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    const T pi = p[i];
-    x[i] += alpha * pi;
-    p[i] = r[i] + beta * pi;
+    const T pi = p[i], ri = r[i], xi = x[i];  // all loads before the stores
+    x[i] = xi + alpha * pi;
+    p[i] = ri + beta * pi;
   }
 }
 

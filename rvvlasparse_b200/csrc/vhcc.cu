@@ -259,7 +259,7 @@ vhcc_spmv_kernel(int64_t NT, int n_eor, int n_rows, const int* __restrict__ thr,
 
 // overflow rows into last_row, in thread order (the reference's atomic add)
 template <class CT>
-__global__ void vhcc_overflow_kernel(int64_t NT, int64_t m, const int* __restrict__ thr, CT* __restrict__ tmp) {
+__global__ void vhcc_overflow_kernel(int64_t NT, int64_t m, const int* __restrict__ thr, CT* tmp) {
   grid_chain();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= NT) return;
@@ -272,7 +272,7 @@ __global__ void vhcc_overflow_kernel(int64_t NT, int64_t m, const int* __restric
 }
 
 template <class X, class CT>
-__global__ void vhcc_out_kernel(int64_t m, const CT* __restrict__ tmp, X* __restrict__ y, X alpha, X beta) {
+__global__ void vhcc_out_kernel(int64_t m, const CT* tmp, X* y, X alpha, X beta) {
   grid_chain();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) write_row(y, (int)i, alpha, beta, (X)tmp[i]);
