@@ -89,6 +89,19 @@ cudaMemPool_t scratch_pool() {
   return pool;
 }
 
+// The device's pool if it has been made.
+static cudaMemPool_t made_pool(int dev) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  return (int)g_pools.size() > dev ? g_pools[(size_t)dev] : nullptr;
+}
+
+bool trim_scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const cudaMemPool_t pool = made_pool(dev);
+  return pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+}
+
 }  // namespace rvvla
 
 extern "C" {
@@ -133,11 +146,7 @@ int rvvla_device_info(int* cc_major, int* cc_minor, int* sms) {
 int rvvla_trim_scratch(void) {
   int dev = 0;
   RVVLA_CUDA(cudaGetDevice(&dev));
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(rvvla::g_pool_mu);
-    if ((int)rvvla::g_pools.size() > dev) pool = rvvla::g_pools[(size_t)dev];
-  }
+  const cudaMemPool_t pool = rvvla::made_pool(dev);
   if (pool) RVVLA_CUDA(cudaMemPoolTrimTo(pool, 0));
   return RVVLA_OK;
 }

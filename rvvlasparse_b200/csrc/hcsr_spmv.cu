@@ -870,9 +870,15 @@ int hcsr_spmv_impl(const rvvla_hcsr* A, X alpha, const X* x, X beta, X* y, cudaS
   // block rows too tall for shared memory: the accumulators are a global
   // scratch array (each CTA owns its slice)
   const size_t smem_g = HLayout<SA>(0).total;
-  const int split = hcsr_split(A, smem_g);
+  int split = hcsr_split(A, smem_g);
   Scratch sc;
-  RVVLA_CUDA(sc.alloc_kept((size_t)split * A->m * sizeof(SA), st));
+  cudaError_t e = sc.alloc_kept((size_t)split * A->m * sizeof(SA), st);
+  if (e == cudaErrorMemoryAllocation && split > 1) {  // no room for a slice per part: one part
+    cudaGetLastError();
+    split = 1;
+    e = sc.alloc_kept((size_t)A->m * sizeof(SA), st);
+  }
+  RVVLA_CUDA(e);
   return vec ? hcsr_launch<V, X, SA, MIX, true, true, true>(A, split, alpha, x, beta, y, sc.as<SA>(), smem_g, st)
              : hcsr_launch<V, X, SA, MIX, false, true, true>(A, split, alpha, x, beta, y, sc.as<SA>(), smem_g, st);
 }

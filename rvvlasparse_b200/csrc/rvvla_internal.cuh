@@ -53,6 +53,8 @@ inline void prefer_shared(K kernel) {
 // The current device's pool for temporary buffers, made on first use; null if
 // it could not be made.
 cudaMemPool_t scratch_pool();
+// Gives back what that pool keeps unused; false if there is none or it fails.
+bool trim_scratch_pool();
 
 // A launch chained to the stream's previous kernel if `chained`.
 #define RVVLA_CHAIN(chained, kernel, blocks, threads, st, ...)                                        \
@@ -78,13 +80,21 @@ struct Scratch {
   cudaStream_t s = nullptr;
   cudaError_t alloc(size_t bytes, cudaStream_t st) {
     s = st;
-    return cudaMallocAsync(&p, bytes == 0 ? 16 : bytes, st);
+    cudaError_t e = cudaMallocAsync(&p, bytes == 0 ? 16 : bytes, st);
+    if (e == cudaErrorMemoryAllocation && trim_scratch_pool()) {  // without what the library's pool keeps
+      cudaGetLastError();
+      e = cudaMallocAsync(&p, bytes == 0 ? 16 : bytes, st);
+    }
+    return e;
   }
   cudaError_t alloc_kept(size_t bytes, cudaStream_t st) {
     cudaMemPool_t pool = bytes <= kScratchKeep ? scratch_pool() : nullptr;
     if (!pool) return alloc(bytes, st);
     s = st;
-    return cudaMallocFromPoolAsync(&p, bytes == 0 ? 16 : bytes, pool, st);
+    const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes == 0 ? 16 : bytes, pool, st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    return alloc(bytes, st);
   }
   ~Scratch() {
     if (p) cudaFreeAsync(p, s);
