@@ -215,14 +215,15 @@ int hcsr_build_impl(const rvvla_crs* src, int vb, int64_t R, int64_t C, double p
   RVVLA_CUDA(cudaMemsetAsync(out->row_ptr, 0, (size_t)std::max<int64_t>(accRows, 1) * sizeof(uint32_t), st));
   h.row_ptr_len = accRows;
   if (b_m > 0 && nz > 0) {
-    const bool smem = b_n * (int64_t)sizeof(int) <= 200 * 1024;
+    constexpr int kShmMax = 200 * 1024;
+    const bool smem = b_n * (int64_t)sizeof(int) <= kShmMax;
     Scratch s_cur;
     if (!smem) RVVLA_CUDA(s_cur.alloc((size_t)nblocks * sizeof(int), st));
     const size_t shm = smem ? (size_t)b_n * sizeof(int) : 0;
 #define HCSR_SCATTER(VB, SM)                                                                                   \
   do {                                                                                                         \
     auto k_ = hcsr_scatter_kernel<VB, SM>;                                                                     \
-    if (shm > 48 * 1024) RVVLA_CUDA(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm)); \
+    if (shm > 48 * 1024) RVVLA_CUDA(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize, kShmMax)); \
     k_<<<(unsigned)b_m, 32, shm, st>>>(m, R, C, b_n, src->Rst, src->Col, (const uint8_t*)src->Val,            \
                                         out->block_ptr, out->row_offset, kind, s_cur.as<int>(), out->col_idx,  \
                                         (uint8_t*)out->values, out->row_ptr);                                  \

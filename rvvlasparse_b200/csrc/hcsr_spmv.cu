@@ -823,7 +823,10 @@ int hcsr_split(const rvvla_hcsr* A, size_t smem) {
 template <class V, class X, class SA, bool MIX, bool VEC, bool GACC, bool SPLIT>
 int hcsr_launch(const rvvla_hcsr* A, int split, X alpha, const X* x, X beta, X* y, SA* gacc, size_t smem, cudaStream_t st) {
   auto kern = hcsr_spmv_kernel<V, X, SA, MIX, VEC, GACC, SPLIT>;
-  RVVLA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the kernel's limit is common to all threads that launch it: always the
+  // largest, not this call's, which another thread's smaller one could replace
+  // before the launch
+  RVVLA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHSmemMax));
   // shared memory for kHMinBlocks CTAs (1 KB of each is the system's), the
   // rest of the SM's 256 KB as L1: the gathers of x hit there.  The SM takes
   // one of a few sizes, and a wish above one of them gets the next.

@@ -154,7 +154,8 @@ int vnec_spmv_impl(const rvvla_vnec* A, X alpha, const X* x, X beta, X* y, cudaS
   const int NT = A->NUM_THREADS_VNEC;
   const size_t xbytes = (size_t)(A->max_nec + A->nLanes) * sizeof(X);
   if (A->vnec_t == 0 || A->vnec_t == 1) {
-    if (xbytes > 200 * 1024)
+    constexpr int kXMax = 200 * 1024;
+    if (xbytes > kXMax)
       return fail(RVVLA_ERR_UNSUPPORTED, "vnec: a thread's compacted x exceeds 200 KB of shared memory; build with more threads");
     if (A->vnec_t == 0) {
       Scratch sc;
@@ -162,7 +163,7 @@ int vnec_spmv_impl(const rvvla_vnec* A, X alpha, const X* x, X beta, X* y, cudaS
       int* crow = sc.as<int>();
       CT* cval = reinterpret_cast<CT*>(sc.as<char>() + ((size_t)NT * sizeof(int) + 255) / 256 * 256);
       auto k_ = vnec_d_kernel<V, X, CT>;
-      if (xbytes > 48 * 1024) RVVLA_CUDA(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xbytes));
+      if (xbytes > 48 * 1024) RVVLA_CUDA(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize, kXMax));
       k_<<<NT, kVnecThreads, xbytes, st>>>(A->m, A->nLanes, A->ptr, (const V*)A->val, A->thread_coord_start,
                                            A->thread_coord_end, A->ecr_indices, A->NEC_NUM, A->use_x_ptr,
                                            A->use_x_indices, A->v_row_ptr, A->col_start, (const V*)A->val_align, x,
@@ -172,7 +173,7 @@ int vnec_spmv_impl(const rvvla_vnec* A, X alpha, const X* x, X beta, X* y, cudaS
       RVVLA_LAUNCHED("merge_fixup_kernel");
     } else {
       auto k_ = vnec_s_kernel<V, X, CT>;
-      if (xbytes > 48 * 1024) RVVLA_CUDA(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xbytes));
+      if (xbytes > 48 * 1024) RVVLA_CUDA(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize, kXMax));
       k_<<<NT, kVnecThreads, xbytes, st>>>(A->nLanes, A->NEC_NUM, A->use_x_ptr, A->use_x_indices, A->tasks,
                                            A->task_start, A->task_end, A->spvv_len, A->row_begin, A->row_end,
                                            A->reorder_col, (const V*)A->reorder_nnz, x, y, alpha, beta);
