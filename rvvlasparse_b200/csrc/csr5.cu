@@ -728,6 +728,7 @@ int csr5_spmv_impl(const rvvla_csr5* A, X alpha, const X* x, X beta, X* y, cudaS
     int* cal_row = cal_row_buf;
     if (!cal) {
       const size_t cal_bytes = (size_t)nwarps * (sizeof(CT) + sizeof(int)) + 256;
+      // fp64: from the device's default pool, as documented (callers watch it there)
       RVVLA_CUDA(sizeof(V) == 8 ? sc.alloc(cal_bytes, st) : sc.alloc_kept(cal_bytes, st));
       cal = sc.as<CT>();
       cal_row = reinterpret_cast<int*>(sc.as<char>() + ((size_t)nwarps * sizeof(CT) + 255) / 256 * 256);
