@@ -135,7 +135,7 @@ __device__ __forceinline__ void store_n(T* p, const T (&v)[N], T alpha, T beta) 
 }
 
 // X rows are gathered 16 bytes a lane (k > 1).
-template <class T, int K, bool VEC>
+template <class T, int K>
 struct XRows {
   static constexpr int VPL = K == 1 ? 1 : 16 / (int)sizeof(T);  // values per lane
   static constexpr int G = K / VPL;                             // lanes per nonzero
@@ -205,7 +205,7 @@ constexpr int kStageNnz = 2048;  // nonzeros of a k > 1 CSR tile staged in share
 template <class T, int K, bool VEC>
 __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restrict__ srst, int* __restrict__ s_col,
                        T* __restrict__ s_val, const T* __restrict__ X, T* __restrict__ Y, T alpha, T beta) {
-  using XR = XRows<T, K, VEC>;
+  using XR = XRows<T, K>;
   constexpr int VPL = XR::VPL, G = XR::G, U = 4;
   const int spr = t.spr, lanes = G * spr, nslots = kBThreads / lanes;
   const int part = threadIdx.x % G, slot = (threadIdx.x / G) % spr, sub = threadIdx.x / lanes;
@@ -305,7 +305,7 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
 template <class T, int K, bool VEC>
 __device__ __forceinline__ void sell_slice(const BatchMat& A, int sl, const T* __restrict__ x, T* __restrict__ Y,
                                            T alpha, T beta, uint64_t pf, uint64_t pl) {
-  using XR = XRows<T, K, VEC>;
+  using XR = XRows<T, K>;
   constexpr int VPL = XR::VPL, G = XR::G;
   constexpr bool BLOCKS = K > 1 && K * sizeof(T) < 256;
   constexpr int U = G <= 4 ? 8 : 4;

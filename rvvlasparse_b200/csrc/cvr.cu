@@ -199,41 +199,36 @@ constexpr int kCvrSplit = 8;
 constexpr int kCvrBatch = 8;
 
 template <class V, class X, class CT>
-__global__ void __launch_bounds__(256, sizeof(V) >= 8 ? 3 : 4)
+__global__ void __launch_bounds__(32 * kCvrSplit, sizeof(V) >= 8 ? 3 : 4)
 cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ vals,
                 const uint32_t* __restrict__ cols, const int* __restrict__ rec, const int* __restrict__ wb,
                 const X* __restrict__ x, X* y, X alpha) {
   constexpr int kCvrU = kCvrBatch;
-  constexpr int kRanges = 8 / kCvrSplit;  // ranges per CTA
-  __shared__ int s_row[8][kCvrU][kS];
-  __shared__ int s_head_row[8][kS];  // per share and lane: row of the first flush (-1: none), the sum
-  __shared__ CT s_head[8][kS];       // before it, and the sum after the last one
-  __shared__ CT s_tail[8][kS];
+  __shared__ int s_row[kCvrSplit][kCvrU][kS];
+  __shared__ int s_head_row[kCvrSplit][kS];  // per share and lane: row of the first flush (-1: none), the sum
+  __shared__ CT s_head[kCvrSplit][kS];       // before it, and the sum after the last one
+  __shared__ CT s_tail[kCvrSplit][kS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t t = (int64_t)blockIdx.x * kRanges + w / kCvrSplit;
-  const int part = w % kCvrSplit;
+  const int64_t t = blockIdx.x;  // the CTA's range
+  const int part = w;
   const bool last = part == kCvrSplit - 1;
-  int64_t vb = 0, ve = 0, rb = 0, re = 0;
-  if (t < NT) {
-    vb = wb[t * (kS + 2)];
-    rb = wb[t * (kS + 2) + 1];
-    ve = (t + 1 < NT) ? wb[(t + 1) * (kS + 2)] : nItems / kS;
-    re = (t + 1 < NT) ? wb[(t + 1) * (kS + 2) + 1] : nrec;
-    const int64_t nv = ve - vb;
-    ve = vb + nv * (part + 1) / kCvrSplit;
-    vb += nv * part / kCvrSplit;
-    if (part > 0) {  // first record at or after the share's first vector: rec[2 * rb] < it <= rec[2 * hi]
-      int64_t lo = rb - 1, hi = re;
-      while (hi - lo > 1) {
-        const int64_t step = (hi - lo + kS - 1) / kS;
-        const int64_t at = lo + step * (lane + 1);
-        const bool before = at < hi && rec[2 * at] < vb * kS;
-        const int k = __popc(__ballot_sync(0xffffffffu, before));  // positions rise: a prefix of the lanes
-        hi = min(hi, lo + step * (k + 1));
-        lo += step * k;
-      }
-      rb = hi;
+  int64_t vb = wb[t * (kS + 2)], rb = wb[t * (kS + 2) + 1];
+  int64_t ve = (t + 1 < NT) ? wb[(t + 1) * (kS + 2)] : nItems / kS;
+  const int64_t re = (t + 1 < NT) ? wb[(t + 1) * (kS + 2) + 1] : nrec;
+  const int64_t nv = ve - vb;
+  ve = vb + nv * (part + 1) / kCvrSplit;
+  vb += nv * part / kCvrSplit;
+  if (part > 0) {  // first record at or after the share's first vector: rec[2 * rb] < it <= rec[2 * hi]
+    int64_t lo = rb - 1, hi = re;
+    while (hi - lo > 1) {
+      const int64_t step = (hi - lo + kS - 1) / kS;
+      const int64_t at = lo + step * (lane + 1);
+      const bool before = at < hi && rec[2 * at] < vb * kS;
+      const int k = __popc(__ballot_sync(0xffffffffu, before));  // positions rise: a prefix of the lanes
+      hi = min(hi, lo + step * (k + 1));
+      lo += step * k;
     }
+    rb = hi;
   }
   const uint64_t pf = policy_evict_first(), pl = policy_evict_last();
   CT res = 0;
@@ -333,7 +328,7 @@ cvr_spmv_kernel(int64_t NT, int64_t nItems, int64_t nrec, const V* __restrict__ 
   }
   s_tail[w][lane] = res;
   __syncthreads();
-  if (part != 0 || t >= NT) return;
+  if (part != 0) return;
   // rows that cross shares: the pieces of a lane in share order
   CT sum = res;
   for (int i = 1; i < kCvrSplit; ++i) {
@@ -370,7 +365,7 @@ int cvr_spmv_impl(const rvvla_cvr* A, X alpha, const X* x, X beta, X* y, cudaStr
   RVVLA_LAUNCHED("cvr_scale_kernel");
   const int64_t NT = A->Nthreads_avail;
   const int64_t nrec = (A->n_record - 2) / 2;
-  RVVLA_CHAIN(true, (cvr_spmv_kernel<V, X, CT>), (NT * kCvrSplit + 7) / 8, 256, st, NT, A->nItems, nrec,
+  RVVLA_CHAIN(true, (cvr_spmv_kernel<V, X, CT>), NT, 32 * kCvrSplit, st, NT, A->nItems, nrec,
               (const V*)A->vPack_vec_vals, A->vPack_vec_cols, A->vPack_vec_record, A->writeback_pos_record, x, y, alpha);
   return RVVLA_OK;
 }

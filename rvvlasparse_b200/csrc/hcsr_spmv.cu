@@ -854,7 +854,6 @@ int hcsr_launch(const rvvla_hcsr* A, int split, X alpha, const X* x, X beta, X* 
 
 template <class V, class X, class SA, bool MIX>
 int hcsr_spmv_impl(const rvvla_hcsr* A, X alpha, const X* x, X beta, X* y, cudaStream_t st) {
-  using P = typename HTypes<V, X, SA, MIX>::P;
   int rc = hcsr_validate(A, x, y);
   if (rc) return rc;
   if (A->m == 0) return RVVLA_OK;
