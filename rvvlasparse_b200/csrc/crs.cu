@@ -260,11 +260,15 @@ int crs_spmv_impl(const rvvla_crs* A, X alpha, const X* x, X beta, X* y, cudaStr
       // CTAs of 4 warps, whose slots turn over sooner and whose registers round
       // to one warp per scheduler more (random rows n = 10^6 mean 8 fp64 57.5 ->
       // 55.4 us with 4 warps instead of 8, mean 19 110 -> 105, Laplacian 2048^2
-      // fp64 82 -> 75, stencil 128^3 183 -> 174), but of 8 at the longest span,
-      // where a warp's rows spread far enough that neighbouring warps sharing
-      // L1 count for more (power law 4M fp64: 278 us with 4, 259 with 8, 270
-      // with 32).  Registers capped for 40 or 48 warps per SM: 81 and 85 us on
-      // the Laplacian.
+      // fp64 82 -> 75, stencil 128^3 183 -> 174), but of 8 at the longest span.
+      // There the two kinds of matrix part: with irregular columns neighbouring
+      // warps that share L1 count for more (power law 4M: fp64 278 us with 4, 259
+      // with 8, 270 with 32; fp32 188 and 183), with regular or evenly random
+      // ones they do not (stencil 160^3 fp64 329 with 4, 341 with 8, mixed 225
+      // and 230; random rows n = 2.6 10^6 mean 30 fp64 372 and 391).  nz, all
+      // that is known here, does not tell them apart; 8 serves the irregular ones,
+      // which lose more.  Registers capped for 40 or 48 warps per SM: 81 and 85
+      // us on the Laplacian.
       auto run = [&](auto tpb) -> int {
         constexpr int T = decltype(tpb)::value;
         auto kern = dot    ? (vec ? crs_run_kernel<V, X, Ac, CT, T, true, false, true>

@@ -302,8 +302,12 @@ int vhcc_spmv_impl(const rvvla_vhcc* A, X alpha, const X* x, X beta, X* y, cudaS
   const int64_t NT = A->num_threads;
   // The VHCC threads' warps do equal work, so those that a first wave leaves
   // over take a second one: in fp64, 40 warps per SM where they all fit then
-  // (600K random rows, 5566 warps: 105 us with 32 per SM, 96 with 40; power law
-  // of 642K rows 87 and 78), else 32 (power law of 4M rows: 334 and 380).  CTAs
+  // (600K random rows, 5566 warps: 104 us with 32 per SM, 97 with 40; power law
+  // of 642K rows 88 and 78; stencil 72^3 87 and 70), else 32 (power law of 4M
+  // rows: 334 and 380).  From a second wave on the form that serves each warp
+  // faster wins also where 40 per SM would save a third (64 to 80 per SM: power
+  // law of 1.28M rows 136 and 144, random 1.1M 160 and 168, stencil 90^3 128 and
+  // 118).  CTAs
   // of four warps against eight: fp32 642K rows 55 -> 52 us, fp64 500K 58 -> 56,
   // 4M 334 -> 336.
   const bool dense = sizeof(V) == 8 && NT > 32 * (int64_t)sm_count() && NT <= 40 * (int64_t)sm_count();
