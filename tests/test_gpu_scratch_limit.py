@@ -10,6 +10,15 @@ import rvvlasparse_b200 as R
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _give_back():
+    """The memory that the test's tensors took, back from torch's cache: the
+    library's builders of later tests allocate outside it."""
+    yield
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+
+
 def _mv(A, x, y):
     st = R.sparse_mv(R.SPARSE_OPERATION_NON_TRANSPOSE, 1.0, A, R.sparse_matrix_descr(), x, 0.0, y)
     return st.code
@@ -43,4 +52,3 @@ def test_tall_block_rows_fall_back_to_one_part():
     del hold
     assert code == 0, msg
     assert torch.equal(y, ref)
-

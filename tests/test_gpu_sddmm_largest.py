@@ -10,6 +10,15 @@ import rvvlasparse_b200 as R
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _give_back():
+    """The memory that the test's tensors took, back from torch's cache: the
+    library's builders of later tests allocate outside it."""
+    yield
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+
+
 def test_largest_pattern():
     nz, m, n = 2 ** 31 - 1, 300_007, 1_000_003
     if torch.cuda.mem_get_info()[0] < 40 << 30:
