@@ -45,8 +45,8 @@
 //           row read them from there and gather X, shuffle reduction over the
 //           groups (same batch: k = 4 918 -> 755, k = 8 1293 -> 930, k = 32 3159 ->
 //           1767 us against k lanes of one value each).  Each group keeps two
-//           sums and adds four products at a time to one of them in turn, so
-//           that a row's error is no larger than that of eight sums (2 and
+//           sums and adds four products at a time to one of them in turn (rows
+//           of 256 bytes: four sums, of one product each), so that a row's error is no larger than that of eight sums (2 and
 //           1000 nonzeros a row, fp32, relative error: 3.6e-7 with two sums
 //           that take the products one by one, 1.8e-7 with eight, 8.5e-8 now).
 #include <algorithm>
@@ -229,10 +229,18 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
     const int rr = it * nslots + sub;
     const bool valid = rr < t.count;
     // the steps' sums go to two accumulators in turn: no chain of roundings is
-    // longer than an eighth of the row and a few
-    T acc[2][VPL];
+    // longer than an eighth of the row and a few.  Rows of 256 bytes (at most
+    // two groups) take one accumulator per product of a step: as short, and the
+    // serial sum of a step is what small batches waited for (100 matrices of 1K
+    // to 8K rows, fp64, k = 32: 323 us with it, 282; 400 of 1K to 4K 859 and 772;
+    // two sums that take the products one by one, less exact, 265 and 720; but
+    // 256 of 1K to 64K 3215, 3999 and 3540)
+    constexpr int P = G >= 16 ? U : 2;
+    T acc[P][VPL];
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) acc[0][i] = acc[1][i] = T(0);
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) acc[p][i] = T(0);
     auto add_step = [&](const T (&t)[VPL]) {
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
@@ -247,7 +255,7 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
       // rows of 128 bytes and more: whole steps, then one nonzero at a time (a
       // repeated row would cost as much as a new one); narrower ones: idle
       // loads of the last step repeat its first entry
-#pragma unroll(G >= 8 ? 2 : 1)
+#pragma unroll(G == 8 ? 2 : 1)
       for (; G >= 8 ? j + (U - 1) * spr < e : j < e; j += U * spr) {
         T v[U];
         alignas(16) T xv[U][VPL];
@@ -258,16 +266,23 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
           v[u] = staged ? s_val[k] : val[b0 + k];
           gather_n<T, VPL, VEC>(x + (int64_t)c * K, xv[u], pl);
         }
-        T t[VPL];
+        if constexpr (P == U) {
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) t[i] = v[0] * xv[0][i];
+          for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int u = 1; u < U; ++u)
-          if (G >= 8 || j + u * spr < e) {
+            for (int i = 0; i < VPL; ++i) acc[u][i] += v[u] * xv[u][i];
+        } else {
+          T t[VPL];
 #pragma unroll
-            for (int i = 0; i < VPL; ++i) t[i] += v[u] * xv[u][i];
-          }
-        add_step(t);
+          for (int i = 0; i < VPL; ++i) t[i] = v[0] * xv[0][i];
+#pragma unroll
+          for (int u = 1; u < U; ++u)
+            if (G >= 8 || j + u * spr < e) {
+#pragma unroll
+              for (int i = 0; i < VPL; ++i) t[i] += v[u] * xv[u][i];
+            }
+          add_step(t);
+        }
       }
       T t[VPL];
 #pragma unroll
@@ -284,7 +299,10 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
     }
     alignas(16) T s[VPL];
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) s[i] = acc[0][i] + acc[1][i];
+    for (int i = 0; i < VPL; ++i) {
+      if constexpr (P == 4) s[i] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
+      else s[i] = acc[0][i] + acc[1][i];
+    }
     for (int off = lanes >> 1; off >= G; off >>= 1)
 #pragma unroll
       for (int i = 0; i < VPL; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], off);
