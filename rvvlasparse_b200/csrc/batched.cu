@@ -58,6 +58,7 @@
 #include <vector>
 
 #include "batched_plan.h"
+#include "batched_tune.h"
 #include "rvvla_internal.cuh"
 
 namespace rvvla {
@@ -839,42 +840,37 @@ int rvvla_batched_autotune(const rvvla_crs* mats, int64_t count, int val_bytes, 
     while (g + 1 < kGroups && avg >= (double)(2 << g)) ++g;
     groups[(size_t)g].push_back(i);
   }
-  struct Cand {
-    int32_t mode, param;
-  };
-  std::vector<Cand> cands;
+  std::vector<TuneCand> cands;
   if (k == 1)
     for (int t = 1; t <= 32; t <<= 1) cands.push_back({0, t});
   else
     cands.push_back({0, 0});
   cands.push_back({1, 32});
   cands.push_back({1, 256});
+  std::vector<TuneCand> pick;
   double total = 0.0;
-  for (const auto& grp : groups) {
-    if (grp.empty()) continue;
-    std::vector<rvvla_crs> sub;
-    for (int64_t i : grp) sub.push_back(mats[i]);
-    double best = 1e30;
-    Cand pick = cands[0];
-    for (const Cand& c : cands) {
-      std::vector<int32_t> md(sub.size(), c.mode), pr(sub.size(), c.param);
-      rvvla_batch_owned plan;
-      int rc = rvvla_batched_plan(sub.data(), (int64_t)sub.size(), val_bytes, k, md.data(), pr.data(), &plan, stream);
-      if (rc) return rc;
-      double ms = 0.0;
-      rc = time_plan(plan.h, st, &ms);
-      rvvla_batched_free(&plan);
-      if (rc) return rc;
-      if (ms < best) {
-        best = ms;
-        pick = c;
-      }
-    }
-    for (int64_t i : grp) {
-      mode[i] = pick.mode;
-      param[i] = pick.param;
-    }
-    total += best;
+  const int rc = tune_layouts(
+      groups, count, cands,
+      [&](const std::vector<int64_t>& ids, const std::vector<TuneCand>& of, double* ms) {
+        std::vector<rvvla_crs> sub;
+        std::vector<int32_t> md, pr;
+        for (size_t i = 0; i < ids.size(); ++i) {
+          sub.push_back(mats[ids[i]]);
+          md.push_back(of[i].mode);
+          pr.push_back(of[i].param);
+        }
+        rvvla_batch_owned plan;
+        int r = rvvla_batched_plan(sub.data(), (int64_t)sub.size(), val_bytes, k, md.data(), pr.data(), &plan, stream);
+        if (r) return r;
+        r = time_plan(plan.h, st, ms);
+        rvvla_batched_free(&plan);
+        return r;
+      },
+      pick, &total);
+  if (rc) return rc;
+  for (int64_t i = 0; i < count; ++i) {
+    mode[i] = pick[(size_t)i].mode;
+    param[i] = pick[(size_t)i].param;
   }
   if (tuned_ms) *tuned_ms = total;
   return RVVLA_OK;
