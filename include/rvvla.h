@@ -647,7 +647,7 @@ int rvvla_autotune(int format, const rvvla_crs* src, int val_type, int mixed, in
  * with 1..32 threads per row for k = 1 or k lanes per row otherwise;
  * SELL-C-sigma with sigma 32 or 256) and writes the fastest per matrix into
  * mode[] / param[] (count entries each), ready for rvvla_batched_plan.  Where
- * that mixes both layouts in a short batch (0.5 ms), the whole batch is timed
+ * that mixes both layouts in a short batch (0.1 ms), the whole batch is timed
  * so, all in CSR and all in SELL, and the fastest of the three is written.
  * *tuned_ms (may be NULL) receives the sum of the groups' best times, or that
  * whole batch's time. */

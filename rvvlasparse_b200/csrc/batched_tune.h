@@ -13,8 +13,9 @@ struct TuneCand {
   int32_t mode, param;  // mode: 0 CSR, 1 SELL
 };
 
-// Batches of up to this time in all are compared whole.
-constexpr double kTuneWholeMs = 0.5;
+// Batches of up to this time in all are compared whole (a second launch, 4 to 8
+// us, counts for little in longer ones).
+constexpr double kTuneWholeMs = 0.1;
 
 // Times every candidate on each group of matrices and gives the group its
 // fastest.  time(ids, cands, &ms) times the matrices `ids` with a candidate each
@@ -22,8 +23,8 @@ constexpr double kTuneWholeMs = 0.5;
 // two launches, which groups timed by themselves do not show (16 matrices of 1K to
 // 4K rows, fp64, k = 1: 22 us with 7 of them in SELL, 14 with all in CSR): a
 // short batch is then timed whole, so and with each group's fastest CSR and
-// fastest SELL candidate.  Longer ones hide the launch and would pay for the
-// plans.  The cands hold both layouts.
+// fastest SELL candidate.  For longer ones that would only lengthen the tuning (256
+// matrices of 1K to 64K rows, k = 1, of 258 us: 0.4 s for the three plans).  The cands hold both layouts.
 template <class Time>
 int tune_layouts(const std::vector<std::vector<int64_t>>& groups, int64_t count, const std::vector<TuneCand>& cands,
                  Time time, std::vector<TuneCand>& out, double* total) {

@@ -58,7 +58,7 @@ def tune(tmp_path_factory):
 
 
 @pytest.mark.parametrize("seed", range(8))
-@pytest.mark.parametrize("scale", [0.001, 0.1])  # ms per matrix: batches well below and above half a millisecond
+@pytest.mark.parametrize("scale", [0.001, 0.1])  # ms per matrix: batches well below and above a tenth of a millisecond
 def test_layouts(tune, seed, scale):
     rng = np.random.default_rng(seed)
     count, launch = 24, 0.006
