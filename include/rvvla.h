@@ -562,7 +562,7 @@ int rvvla_sddmm_values_f32(const rvvla_crs* A, const float* g, const float* x, f
 
 /* ------------------------------------------------------------ batched
  * No reference counterpart.  Many independent matrices, each with k right-
- * hand sides, in one persistent launch per layout (CSR, SELL): Y_i = alpha * A_i X_i + beta * Y_i.
+ * hand sides, in one launch per layout (CSR, SELL): Y_i = alpha * A_i X_i + beta * Y_i.
  * X_i is n_i x k and Y_i is m_i x k, row-major, packed matrix after matrix
  * (matrix i starts at x_off[i] / y_off[i] elements). */
 typedef struct rvvla_batch {
@@ -592,7 +592,7 @@ typedef struct rvvla_batch_owned {
 int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int k, const int32_t* mode,
                        const int32_t* param, rvvla_batch_owned* out, void* stream);
 void rvvla_batched_free(rvvla_batch_owned* b);
-/* One persistent launch over all CSR matrices and one over all SELL ones. */
+/* One launch over all CSR matrices and one over all SELL ones. */
 int rvvla_batched_spmv_f64(const rvvla_batch* B, double alpha, const double* X, double beta, double* Y,
                            void* stream);
 int rvvla_batched_spmv_f32(const rvvla_batch* B, float alpha, const float* X, float beta, float* Y,

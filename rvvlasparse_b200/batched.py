@@ -1,5 +1,5 @@
 """Batched SpMV over many CRS matrices with k right-hand sides, in one
-persistent launch (optionally captured in a CUDA graph), through the C ABI
+launch per layout (optionally captured in a CUDA graph), through the C ABI
 (``rvvla_batched_*``).  No reference counterpart.
 
 X holds every matrix's n_i x k block and Y every m_i x k block, row-major,

@@ -4,7 +4,7 @@
 //
 // Plan (rvvla_batched_plan): each matrix runs either as CSR (the caller's
 // arrays) or as SELL-C-sigma (C = 32, built on the GPU and owned by the
-// plan).  All CSR matrices are one persistent launch over a list of tiles of
+// plan).  All CSR matrices are one launch over a list of tiles of
 // bounded work, all SELL matrices another over shares of slices; a plan of one
 // layout is one launch.
 //
@@ -36,8 +36,8 @@
 // tiles of slices over all the CTAs that fit: k = 1 468 -> 242, k = 4 1024 ->
 // 510, k = 8 2602 -> 582, k = 32 16738 -> 1495 us.
 //
-// CSR kernel: a persistent grid of all the CTAs that fit walks the tiles with
-// a grid stride;
+// CSR kernel: several waves of the CTAs that fit walk the tiles with a grid
+// stride (kCsrWaves);
 //   k = 1   tpr lanes per row (tpr in {1,2,4,...,32}, per matrix): lanes
 //           stride over the row, shuffle reduction inside the group;
 //   k > 1   the tile's columns and values (at most 2048 nonzeros) are staged in
@@ -234,8 +234,7 @@ __device__ void csr_kn(const BatchMat& A, const BatchTile& t, const int* __restr
     // two groups) take one accumulator per product of a step: as short, and the
     // serial sum of a step is what small batches waited for (100 matrices of 1K
     // to 8K rows, fp64, k = 32: 323 us with it, 282; 400 of 1K to 4K 859 and 772;
-    // two sums that take the products one by one, less exact, 265 and 720; but
-    // 256 of 1K to 64K 3215, 3999 and 3540)
+    // two sums that take the products one by one, less exact, 265 and 720)
     constexpr int P = G >= 16 ? U : 2;
     T acc[P][VPL];
 #pragma unroll
@@ -479,6 +478,16 @@ batched_kernel(int64_t ntiles, const BatchTile* __restrict__ tiles, const BatchM
 }
 
 constexpr int64_t kTileWork = 8192;  // k = 1 CSR tile: nonzeros + rows
+
+// CSR CTAs per resident one, at most; a CTA per tile for X rows of 128 bytes and
+// more.  CTAs that walk a long list with a grid stride drift apart and spread over
+// more matrices than L2 holds the X of; new CTAs take the tiles in order.  1024
+// matrices of 1K to 64K rows, k = 32, fp32: 11.7 ms with the resident CTAs, 10.6,
+// 8.3 and 7.6 with 4 and 16 times as many and one per tile; 256 of them, fp64, 4.0,
+// 3.8, 3.0, 2.8 ms.  Narrower rows gain less and lose a little to a CTA per tile
+// (256, fp32: k = 1 533, 516, 489, 484 us, k = 4 751, 756, 742, 759, k = 8 923,
+// 947, 915, 934).
+constexpr int64_t kCsrWaves = 16;
 
 int default_tpr(double avg) {
   int t = 1;
@@ -759,9 +768,11 @@ int rvvla_batched_plan(const rvvla_crs* mats, int64_t count, int val_bytes, int 
     to += l.second;
   }
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, "cudaStreamSynchronize");
-  // persistent grid of the CSR kernel: every SM filled with as many CTAs as fit
+  // grid of the CSR kernel: every SM filled with as many CTAs as fit, some times over
   const int per_sm = (val_bytes == 8) ? resident_ctas<double>(k) : resident_ctas<float>(k);
-  h.grid = (int32_t)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count() * per_sm, (int64_t)tiles.size()));
+  // (kCsrWaves)
+  const int64_t most = k * val_bytes >= 128 ? INT32_MAX : (int64_t)sm_count() * per_sm * kCsrWaves;
+  h.grid = (int32_t)std::max<int64_t>(1, std::min<int64_t>(most, (int64_t)tiles.size()));
   h.block = kBThreads;
   h.mats = out->mats;
   h.tiles = out->tiles;
