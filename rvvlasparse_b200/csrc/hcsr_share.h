@@ -1,7 +1,8 @@
-// hcsr_share.h — the part of a window's COO stream that one CTA of a block row
-// takes (hcsr_spmv.cu), in host and device code.
+// hcsr_share.h — how many CTAs share a block row and which part of a window's
+// COO stream each of them takes (hcsr_spmv.cu), in host and device code.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 
 #include "host_device.h"
@@ -27,6 +28,20 @@ RVVLA_HD inline HcsrShare hcsr_share(int total, int parts, int part) {
   const int64_t lo = share * part < total ? share * part : total;
   const int64_t hi = lo + share < total ? lo + share : total;
   return {(int)lo, (int)hi};
+}
+
+constexpr int64_t kHSplitMax = 8;     // portable cluster size
+constexpr int64_t kHSplitNz = 2048;   // nonzeros of a block row that a part keeps at least
+constexpr int64_t kHSplitBlk = 96;    // nonzeros of a large block that a warp keeps at least
+
+// Parts of a block row: as many as the free CTA slots give, fewer where a part
+// would have too little of the block row, or its `warps` warps of the average
+// block, if that has the `large` nonzeros with which blocks are cut by rows.
+inline int hcsr_parts(int64_t b_m, int64_t b_n, int64_t nz, int64_t slots, int warps, int large) {
+  int64_t s = std::min({slots / b_m, nz / (b_m * kHSplitNz), kHSplitMax});
+  const int64_t block = nz / b_m / std::max<int64_t>(b_n, 1);
+  if (block >= large) s = std::min(s, block / (warps * kHSplitBlk));
+  return (int)std::max<int64_t>(1, s);
 }
 
 }  // namespace rvvla

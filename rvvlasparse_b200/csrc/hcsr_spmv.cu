@@ -801,8 +801,6 @@ int hcsr_validate(const rvvla_hcsr* A, const void* x, const void* y) {
 // static arrays.
 constexpr size_t kHSmemMax = 226 * 1024;
 
-constexpr int64_t kHSplitMax = 8;                           // portable cluster size
-constexpr int64_t kHSplitNz = 2048;                         // nonzeros a part keeps at least
 
 // CTAs per block row: as many as keep all CTAs resident at once (cluster
 // sizes need not be powers of two; an eighth of the slots is left free, since a
@@ -813,11 +811,17 @@ constexpr int64_t kHSplitNz = 2048;                         // nonzeros a part k
 // fewer leave SMs idle (power law, fp64, 100K rows in 50 block rows 67 -> 35
 // us, 300K rows 93 -> 62, 30K rows 60 -> 27; fp32 with R = 4000, 1M rows in 251
 // block rows 166 -> 117; accumulators in scratch, 1M rows, R = 60000, fp64
-// 2317 -> 477).
+// 2317 -> 477).  Blocks that take the row-range path (large ones) are searched by
+// every warp of the block row, so where the average block is one, a warp's share
+// of it is kept at kHSplitBlk nonzeros (hcsr_parts).  Random rows, parts by that
+// rule / by the slots alone / 16-warp CTAs without parts: fp32 n = 357K mean 39
+// 370 / 510 / 367 us (2 and 5 parts), 200K mean 30 193 / 285 / 193 (3, 8), 500K
+// mean 40 502 / 702 / 517 (1, 4); fp64 100K mean 40 205 / 314 / 203 (2, 8), 150K
+// mean 40 333 / 451 / 312 (1, 6).  64 and 128 nonzeros: 366 and 425, 195 and 180,
+// 513 and 502, 222 and 190, 331 and 334.
 int hcsr_split(const rvvla_hcsr* A, size_t smem) {
   const int64_t per_sm = std::min<int64_t>(kHMinBlocks, (kHSmemMax + 2048) / (smem + 2048));
-  const int64_t s = std::min(sm_count() * per_sm * 7 / 8 / A->b_m, A->nz / (A->b_m * kHSplitNz));
-  return (int)std::max<int64_t>(1, std::min(s, kHSplitMax));
+  return hcsr_parts(A->b_m, A->b_n, A->nz, sm_count() * per_sm * 7 / 8, kHW, kHBig);
 }
 
 template <class V, class X, class SA, bool MIX, bool VEC, bool GACC, bool SPLIT>
