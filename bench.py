@@ -525,7 +525,7 @@ def form_precision(torch, pk):
 def form_batched(torch, pk):
     """1,024 independent matrices (n log-uniform in [1024, 65536], average
     nonzeros per row U[4, 64], Poisson rows, uniform columns, fp32 U[-1,1]),
-    k in {1, 4, 8, 32} right-hand sides; autotuned; one persistent launch per
+    k in {1, 4, 8, 32} right-hand sides; autotuned; one launch per layout and
     product, replayed from a CUDA graph.  Bytes = 8*nnz + 4*(m+1) + 4*k*(n+m)
     summed over the matrices."""
     import oracle as O

@@ -43,8 +43,8 @@
 //   k > 1   the tile's columns and values (at most 2048 nonzeros) are staged in
 //           shared memory with one coalesced pass; spr groups of G lanes per
 //           row read them from there and gather X, shuffle reduction over the
-//           groups (same batch: k = 4 918 -> 755, k = 8 1293 -> 930, k = 32 3159 ->
-//           1767 us against k lanes of one value each).  Each group keeps two
+//           groups (same batch: k = 4 918 -> 744, k = 8 1293 -> 916, k = 32 3159 ->
+//           1758 us against k lanes of one value each).  Each group keeps two
 //           sums and adds four products at a time to one of them in turn (rows
 //           of 256 bytes: four sums, of one product each), so that a row's error is no larger than that of eight sums (2 and
 //           1000 nonzeros a row, fp32, relative error: 3.6e-7 with two sums
