@@ -644,7 +644,7 @@ int rvvla_autotune(int format, const rvvla_crs* src, int val_type, int mixed, in
 
 /* Autotuner: groups the matrices by average row length (powers of two),
  * times every candidate configuration on each group with CUDA events (CSR
- * with 1..32 threads per row for k = 1 or k lanes per row otherwise;
+ * with 1..32 threads per row for k = 1, as the plan maps it otherwise;
  * SELL-C-sigma with sigma 32 or 256) and writes the fastest per matrix into
  * mode[] / param[] (count entries each), ready for rvvla_batched_plan.  Where
  * that mixes both layouts in a short batch (0.1 ms), the whole batch is timed
